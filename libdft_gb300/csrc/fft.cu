@@ -19,25 +19,45 @@ struct PlanEntry {
   int radix[FFT_MAX_STAGES];
   void *tw;
 };
-std::map<std::pair<int, int>, PlanEntry> g_plans;   // (n, sizeof(T)) -> plan
+std::map<std::pair<int, int>, PlanEntry> g_plans;   // (n, sizeof(T), + 1 for the small variant) -> plan
 std::mutex g_plan_mu;
 
-// FP64: radices up to 8 (the FP64 kernels compile for those only)
-int factorize_small(int n, int *radix, int *nst) {
-  int m = n, k = 0;
-  while (m % 8 == 0 && m > 8) { radix[k++] = 8; m /= 8; }
-  if (m % 8 == 0) { radix[k++] = 8; m /= 8; }
-  if (m % 4 == 0) { radix[k++] = 4; m /= 4; }
-  if (m % 2 == 0) { radix[k++] = 2; m /= 2; }
-  while (m % 3 == 0) { radix[k++] = 3; m /= 3; }
-  while (m % 5 == 0) { radix[k++] = 5; m /= 5; }
-  if (m != 1 || k > FFT_MAX_STAGES) return DFTGPU_ERR_SIZE;
-  *nst = k;
-  return DFTGPU_OK;
+// FP64 operations per element of a radix-R stage without / with twiddles (the
+// powers of two carry theirs inside the butterfly, the others multiply first)
+struct RadixCost { int r; double first, rest; };
+constexpr RadixCost kRadix[] = { { 16, 9.25, 12 }, { 15, 11.2, 14.9 }, { 12, 8, 11.7 }, { 10, 9.2, 12.8 }, { 9, 9.8, 13.3 },
+                                 { 8, 6.5, 9 }, { 6, 6, 9.3 }, { 5, 7.2, 10.4 }, { 4, 4, 6 }, { 3, 4, 6.7 }, { 2, 2, 3 } };
+constexpr double kStageCost = 6;   // a pass through shared memory, in the same unit: the fewest stages first
+
+// The cheapest product of radices, the untwiddled first stage included in the
+// choice; a small charge on the largest radix prefers 8 x 8 to 16 x 4 (as many
+// butterflies in either stage).  Depth-first over at most FFT_MAX_STAGES stages.
+void search(int m, int cap, int depth, double cost, int big, int *cur, double *best, int *radix, int *nst) {
+  if (m == 1) {
+    if (cost + 0.1 * big < *best) {
+      *best = cost + 0.1 * big;
+      *nst = depth;
+      for (int i = 0; i < depth; i++) radix[i] = cur[i];
+    }
+    return;
+  }
+  if (depth == FFT_MAX_STAGES || cost >= *best) return;
+  for (const RadixCost &k : kRadix)
+    if (m % k.r == 0 && k.r <= cap) {
+      cur[depth] = k.r;
+      search(m / k.r, cap, depth + 1, cost + (depth ? k.rest : k.first) + kStageCost, big > k.r ? big : k.r, cur, best, radix, nst);
+    }
 }
 
-// FP32
-int factorize(int n, int *radix, int *nst) {
+int factorize_fp64(int n, int cap, int *radix, int *nst) {
+  int cur[FFT_MAX_STAGES];
+  double best = 1e9;
+  *nst = 0;
+  search(n, cap, 0, 0.0, 0, cur, &best, radix, nst);
+  return best < 1e9 ? DFTGPU_OK : DFTGPU_ERR_SIZE;
+}
+// FP32: few stages, not bound by operations (16 first: 240^3 12.0 ms in two steps against 13.0 as 15, 16)
+int factorize_fp32(int n, int *radix, int *nst) {
   int m = n, k = 0, a = 0, b = 0, c = 0;
   while (m % 2 == 0) { m /= 2; a++; }
   while (m % 3 == 0) { m /= 3; b++; }
@@ -61,23 +81,30 @@ int factorize(int n, int *radix, int *nst) {
 }
 }  // namespace
 
-template <typename T> int get_plan(int n, FftPlan<T> *plan) {
+int fft_radices(int n, int prec, bool small, int *radix, int *nst) {
+  *nst = 0;
+  if (n == 1) return DFTGPU_OK;
+  return prec == DFTGPU_FP64 ? factorize_fp64(n, small ? 5 : 16, radix, nst) : factorize_fp32(n, radix, nst);
+}
+
+template <typename T> int get_plan(int n, FftPlan<T> *plan, bool small) {
   typedef typename cplx_t<T>::type C;
   if (n < 1 || n > FFT_MAX_LINE) {
     set_error(DFTGPU_ERR_SIZE, "FFT length %d outside [1, %d]", n, FFT_MAX_LINE);
     return DFTGPU_ERR_SIZE;
   }
+  if (sizeof(T) == 4) small = false;   // one FP32 variant
   std::lock_guard<std::mutex> lock(g_plan_mu);
-  auto key = std::make_pair(n, (int) sizeof(T));
+  auto key = std::make_pair(n, (int) sizeof(T) + small);
   auto it = g_plans.find(key);
   if (it == g_plans.end()) {
     PlanEntry e;
-    if (n == 1) { e.nst = 0; }
-    else if ((sizeof(T) == 4 ? factorize(n, e.radix, &e.nst) : factorize_small(n, e.radix, &e.nst)) != DFTGPU_OK) {
+    if (fft_radices(n, sizeof(T) == 8 ? DFTGPU_FP64 : DFTGPU_FP32, small, e.radix, &e.nst) != DFTGPU_OK) {
       set_error(DFTGPU_ERR_SIZE, "FFT length %d is not of the form 2^a 3^b 5^c", n);
       return DFTGPU_ERR_SIZE;
     }
-    C *h = (C *) malloc(sizeof(C) * (size_t) n);
+    const size_t nt = plan_table<T>(n);
+    C *h = (C *) malloc(sizeof(C) * nt);
     for (int t = 0; t < n; t++) {
       // reduce the angle to [-pi, pi] and evaluate in long double, round once
       long tt = (t <= n / 2) ? t : (long) t - n;
@@ -85,6 +112,7 @@ template <typename T> int get_plan(int n, FftPlan<T> *plan) {
       const long double cr = cosl(ang), ci = sinl(ang);
       h[t].x = (T) cr;
       h[t].y = (T) ci;
+      if constexpr (sizeof(T) == 8) h[n + t] = cos_tan((double) cr, (double) ci);
       if (sizeof(T) == 4) {
         // of the float pairs within one ulp of (cos, sin), take the one
         // closest to the unit circle: independent rounding leaves |w|^2 off 1
@@ -101,8 +129,8 @@ template <typename T> int get_plan(int n, FftPlan<T> *plan) {
       }
     }
     void *d = nullptr;
-    cudaError_t err = cudaMalloc(&d, sizeof(C) * (size_t) n);
-    if (err == cudaSuccess) err = cudaMemcpy(d, h, sizeof(C) * (size_t) n, cudaMemcpyHostToDevice);
+    cudaError_t err = cudaMalloc(&d, sizeof(C) * nt);
+    if (err == cudaSuccess) err = cudaMemcpy(d, h, sizeof(C) * nt, cudaMemcpyHostToDevice);
     // the table is complete on the device before any stream (also a
     // non-blocking one: a caller's, or a parallel branch) reads it
     if (err == cudaSuccess) err = cudaDeviceSynchronize();
@@ -121,23 +149,49 @@ template <typename T> int get_plan(int n, FftPlan<T> *plan) {
   return DFTGPU_OK;
 }
 
-template int get_plan<float>(int, FftPlan<float> *);
-template int get_plan<double>(int, FftPlan<double> *);
+template int get_plan<float>(int, FftPlan<float> *, bool);
+template int get_plan<double>(int, FftPlan<double> *, bool);
 
-int choose_tile(int n, int nb, size_t cplx_bytes, int nbufs, int *B, size_t *smem, bool partial) {
-  const size_t budget = 113 * 1024, hard = 225 * 1024;
-  const int cand[5] = { 16, 8, 4, 2, 1 };
-  for (int pass = 0; pass < 2; pass++) {
-    for (int c = 0; c < 5; c++) {
-      int b = cand[c];
-      if (nb % b && !partial) continue;
-      if (b > nb && b > 1) continue;
-      size_t s = (size_t) nbufs * (size_t) n * (size_t) tile_pitch(b) * cplx_bytes;
-      if (s <= (pass == 0 ? budget : hard)) { *B = b; *smem = s; return DFTGPU_OK; }
-    }
+size_t max_smem() {
+  static size_t v = 0;
+  if (!v) {
+    int dev = 0, m = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&m, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess)
+      v = (size_t) m;
   }
-  set_error(DFTGPU_ERR_SIZE, "FFT tile for n=%d does not fit in shared memory", n);
-  return DFTGPU_ERR_SIZE;
+  return v;
+}
+
+// About 16 values per thread (one butterfly of radix 16) at 128 threads in
+// FP64 and 256 in FP32; fewer lines per CTA while the launch would not give
+// every SM four CTAs, down to runs of 64 bytes where a side is strided and in
+// FP64 to one full warp of butterflies (an FP64 warp instruction takes its 16 clocks
+// of the SM's pipe whatever the number of its active lanes).
+int choose_tile(int n, int big, int na, int nb, size_t cplx_bytes, int nbufs, bool strided, size_t table, TileShape *t) {
+  const size_t hard = max_smem();
+  const int most = cplx_bytes == 16 ? 2560 : 5120;
+  int least = strided ? (int) (64 / cplx_bytes) : 1;
+  while (cplx_bytes == 16 && least < 32 && least * n < 32 * big) least *= 2;   // a full warp of the largest butterflies
+  int B = 32;
+  while (B > 1 && (B * n > most || B >= 2 * nb)) B >>= 1;
+  if (B < least) B = least;
+  while (B > 1 && B >= 2 * nb) B >>= 1;
+  while (B > least && (size_t) na * ((nb + B - 1) / B) < (size_t) 4 * rt().num_sms) B >>= 1;
+  auto need = [&](int b) { return (size_t) nbufs * b * Tile::pitch(n) * cplx_bytes + table + (table ? (size_t) b * cplx_bytes : 0); };
+  while (B > 1 && need(B) > hard) B >>= 1;
+  if (need(B) > hard) {
+    set_error(DFTGPU_ERR_SIZE, "FFT tile for n=%d does not fit in shared memory", n);
+    return DFTGPU_ERR_SIZE;
+  }
+  t->B = B;
+  t->logB = 0;
+  while ((1 << t->logB) < B) t->logB++;
+  int th = (B * n / (cplx_bytes == 16 ? 8 : 4) + 31) / 32 * 32;
+  const int cap = cplx_bytes == 16 && B * n <= most ? 128 : 256;
+  t->threads = th < 64 ? 64 : th > cap ? cap : th;
+  t->smem = need(B);
+  return DFTGPU_OK;
 }
 
 bool fused_zy_off() {
@@ -337,18 +391,11 @@ template <typename T> int launch_xconv(XConvArgs<T> &A) {
       if (rc >= 0) return rc;
     }
   }
-  DFT_TRY(get_plan<T>(A.nx, &A.plan));
-  int B; size_t smem;
-  DFT_TRY(choose_tile(A.nx, A.ny, sizeof(C), 3, &B, &smem));   // three tiles (xconv_kernel)
-  A.B = B;
+  DFT_TRY(get_plan<T>(A.nx, &A.plan, small_pass(A.nx, A.nkz, A.ny)));
   A.kxh = A.nx / 2 + 1;
   A.kyh = A.ny / 2 + 1;
-  static bool attr = false;
-  if (!attr) {
-    DFT_CUDA(cudaFuncSetAttribute(xconv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) rt().max_smem_optin));
-    attr = true;
-  }
-  dim3 grid(A.ny / B, A.nkz);
+  A.acc_buf = 0;
+  for (int o = 0; o < A.nout; o++) A.acc_buf |= A.out[o].nt != 1;
   double bytes = 0.0;
   {
     const double spec = (double) A.nkz * A.nx * A.ny * sizeof(C);
@@ -365,7 +412,21 @@ template <typename T> int launch_xconv(XConvArgs<T> &A) {
     }
   }
   ProfScope prof("fft_x_conv", bytes);
-  xconv_kernel<T><<<grid, FFT_THREADS, smem, rt().stream>>>(A);
+  if (A.nx == 1) {
+    xconv_point_kernel<T><<<(A.nkz * A.ny + 127) / 128, 128, 0, rt().stream>>>(A);
+    DFT_CHECK_LAUNCH();
+    return DFTGPU_OK;
+  }
+  TileShape t;
+  DFT_TRY(choose_tile(A.nx, max_radix(A.plan), A.nkz, A.ny, sizeof(C), xconv_bufs(A.plan.nst, A.acc_buf), true, 0, &t));
+  A.B = t.B;
+  A.logB = t.logB;
+  static bool attr = false;
+  if (!attr) {
+    DFT_CUDA(cudaFuncSetAttribute(xconv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) max_smem()));
+    attr = true;
+  }
+  xconv_kernel<T><<<dim3((A.ny + t.B - 1) / t.B, A.nkz), t.threads, t.smem, rt().stream>>>(A);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }
@@ -388,25 +449,9 @@ template <typename T> int launch_xkinetic(KinArgs<T> &A) {
       if (rc >= 0) return rc;
     }
   }
-  DFT_TRY(get_plan<T>(A.nx, &A.plan));
-  int B; size_t smem;
-  DFT_TRY(choose_tile(A.nx, A.ny, sizeof(C), 2, &B, &smem));
-  smem = kin_smem(A.nx, B, sizeof(C));
-  if (smem > rt().max_smem_optin) {
-    set_error(DFTGPU_ERR_SIZE, "kinetic pass for nx=%d does not fit in shared memory", A.nx);
-    return DFTGPU_ERR_SIZE;
-  }
-  A.B = B;
-  static bool attr = false;
-  if (!attr) {
-    DFT_CUDA(cudaFuncSetAttribute(xkinetic_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) rt().max_smem_optin));
-    attr = true;
-  }
-  dim3 grid(A.ny / B, A.nz);
+  DFT_TRY(get_plan<T>(A.nx, &A.plan, small_pass(A.nx, A.nz, A.ny)));
   ProfScope prof("fft_x_kinetic", 2.0 * A.nx * A.ny * A.nz * sizeof(C));
-  xkinetic_kernel<T><<<grid, FFT_THREADS, smem, rt().stream>>>(A);
-  DFT_CHECK_LAUNCH();
-  return DFTGPU_OK;
+  return launch_generic_xkinetic<T>(A, rt().stream);
 }
 
 template int launch_xconv<float>(XConvArgs<float> &);

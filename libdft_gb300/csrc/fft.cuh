@@ -10,10 +10,11 @@
 // row of length nz into nz/2 complex values (even + i odd), one FFT of length
 // nz/2 and a twiddle post-processing step; the inverse does the reverse.
 //
-// The generic line pass (any 2^a 3^b 5^c length, and all of FP64) stages a
-// tile of B lines in shared memory as [n][B+1] (element-major, padded), runs
-// a Stockham autosort FFT (ping-pong buffers; radices {16, 15, 12, 10, 9, 8,
-// 6, 5, 4, 3, 2} in FP32, {8, 5, 4, 3, 2} in FP64) and streams the tile back.  Loads and
+// The generic line pass (any 2^a 3^b 5^c length, and all of FP64) runs a
+// Stockham autosort FFT over a tile of B lines with the butterflies in
+// registers (radices 16, 15, 12, 10, 9, 8, 6, 5, 4, 3, 2): the first stage
+// loads from global memory, the last one stores to it, and shared memory
+// carries the line between stages.  Loads and
 // stores go through functors, which is where pointwise producers (|psi|^2,
 // products of fields, phase factors) and consumers (accumulate into the
 // potential) are fused.  Twiddles come from per-length tables computed in
@@ -38,11 +39,30 @@ template <typename T> struct FftPlan {
   int n;                       // transform length
   int nst;                     // number of stages
   int radix[FFT_MAX_STAGES];
-  const typename cplx_t<T>::type *tw;   // tw[t] = exp(-2 pi i t / n), t < n
+  const typename cplx_t<T>::type *tw;   // tw[t] = exp(-2 pi i t / n), t < n; FP64: tw[n + t] = its (cos, tan)
 };
+// entries of a plan's table
+template <typename T> constexpr size_t plan_table(size_t n) { return sizeof(T) == 8 ? 2 * n : n; }
+// The tangent of a table entry.  A cosine that rounds to zero gets a tiny one
+// in its place, so that cos * tan is still the sine.
+__host__ __device__ __forceinline__ double2 cos_tan(double c, double s) {
+  if (c == 0.0) c = 1e-30;
+  double2 r; r.x = c; r.y = s / c;
+  return r;
+}
 
-// Host: build (and cache) the plan for length n in precision T.
-template <typename T> int get_plan(int n, FftPlan<T> *plan);
+// Radices of a 2^a 3^b 5^c length (DFTGPU_ERR_SIZE otherwise).
+int fft_radices(int n, int prec, bool small, int *radix, int *nst);
+// Host: build (and cache) the plan for length n in precision T.  small: the
+// FP64 variant with radices up to 5.
+template <typename T> int get_plan(int n, FftPlan<T> *plan, bool small = false);
+// FP64 passes of up to 2^19 values run with the small radices: their kernels
+// are over in microseconds and mostly wait for their straight-line code to
+// arrive, and four radix-4 stages take 22 operations an element where two of
+// radix 16 take 21.  Measured on full potentials, radices up to 5 against up
+// to 16 (us): 32^3 291 / 365, 64^3 517 / 541, 96 x 90 x 80 1452 / 1493, 128^3
+// (2^20 values a pass) 3259 / 3230, 160 x 150 x 144 7971 / 7295.
+inline bool small_pass(int n, int na, int nb) { return (size_t) n * na * nb <= (size_t) 1 << 19; }
 
 // ------------------------------------------------------------ butterflies
 template <typename C, typename T>
@@ -195,238 +215,347 @@ __device__ __forceinline__ void small_dft(C *u, T s) {
   }
 }
 
-// One radix-R Stockham stage over a tile of B lines in [n][ldb] layout.
-// FP32: thread t on line t % B, butterflies t / B + j blockDim.x / B; FP64:
-// butterfly (line, index) = (idx % B, idx / B) for idx = t + j blockDim.x,
-// twiddle index mod n.  Each form is the faster one for its precision: the
-// first took the FP32 2.3.5 steps from 94 to 119 steps/s at 240^3, the
-// second the FP64 256^3 step from 99 to 91 ms.
-template <int R, typename T>
-__device__ __forceinline__ void stockham_stage(const typename cplx_t<T>::type *__restrict__ in,
-                                               typename cplx_t<T>::type *__restrict__ out,
-                                               int n, int B, int ldb, int p,
-                                               const typename cplx_t<T>::type *__restrict__ tw, T s) {
-  typedef typename cplx_t<T>::type C;
-  const int nR = n / R, twstep = n / (p * R);
-  auto butterfly = [&](int l, int i, int k, int tq) {
-    C u[R];
-#pragma unroll
-    for (int q = 0; q < R; q++) {
-      C v = in[(i + q * nR) * ldb + l];
-      if (q > 0 && k > 0) {
-        C w = __ldg(&tw[tq ? (q * k * twstep) % n : q * k * twstep]);   // q k twstep < n
-        w.y *= -s;   // tw holds exp(-i...); inverse (s=+1) uses the conjugate
-        v = cmul(v, w);
-      }
-      u[q] = v;
-    }
-    small_dft<R, C, T>(u, s);
-    const int j = (i - k) * R + k;
-#pragma unroll
-    for (int q = 0; q < R; q++) out[(j + q * p) * ldb + l] = u[q];
-  };
-  if constexpr (sizeof(T) == 4) {
-    const int l = threadIdx.x % B, istep = blockDim.x / B;
-    for (int i = threadIdx.x / B; i < nR; i += istep) butterfly(l, i, i % p, 0);
+// A radix-R butterfly of power-of-two R as polynomial evaluation: the R outputs
+// are P(z_j) = sum_q u_q z_j^q at z_j = w omega_R^j, and by even / odd halves
+//   P(z_j), P(z_{j+M/2}) = E(z_j^2) +- z_j O(z_j^2),
+// so each level is one complex a +- z b and the stage twiddle w is part of z.
+// The table values read are 1 + 1 + 2 + 4 for R = 16 (z_{j+M/4} = -i z_j):
+// w^{R/M} omega_M^j, j < M/4, for M = 2, 4, 8, 16.
+// FP64: z = c (1 + i r) with c = cos, r = tan of its angle, so that
+// t = (b.x - r b.y, b.y + r b.x) and a +- c t take six operations where a
+// product by the twiddle followed by the sums takes eight, with two roundings
+// on the way to each output instead of three (t.x c is Re(z b) to one
+// rounding whatever the size of r).  FP32 is not bound by its operations and
+// keeps (cos, sin) pairs rounded to the unit circle.
+__device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
+
+__device__ __forceinline__ void bf_z(float2 &a, float2 &b, float2 z) {   // (a + z b, a - z b)
+  const float2 t = a, v = b;
+  a.x = fmaf(-z.y, v.y, fmaf(z.x, v.x, t.x));
+  a.y = fmaf(z.y, v.x, fmaf(z.x, v.y, t.y));
+  b.x = fmaf(z.y, v.y, fmaf(-z.x, v.x, t.x));
+  b.y = fmaf(-z.y, v.x, fmaf(-z.x, v.y, t.y));
+}
+__device__ __forceinline__ void bf_miz(float2 &a, float2 &b, float2 z) {   // with -i z for z
+  bf_z(a, b, make_float2(z.y, -z.x));
+}
+__device__ __forceinline__ void bf_z(double2 &a, double2 &b, double2 z) {   // z = z.x (1 + i z.y)
+  const double tx = fma(-z.y, b.y, b.x), ty = fma(z.y, b.x, b.y);
+  b.x = fma(-z.x, tx, a.x);
+  b.y = fma(-z.x, ty, a.y);
+  a.x = fma(z.x, tx, a.x);
+  a.y = fma(z.x, ty, a.y);
+}
+__device__ __forceinline__ void bf_miz(double2 &a, double2 &b, double2 z) {
+  const double tx = fma(-z.y, b.y, b.x), ty = fma(z.y, b.x, b.y);
+  b.x = fma(-z.x, ty, a.x);
+  b.y = fma(z.x, tx, a.y);
+  a.x = fma(z.x, ty, a.x);
+  a.y = fma(-z.x, tx, a.y);
+}
+template <typename C> __device__ __forceinline__ void bf_1(C &a, C &b) { const C t = a; a = t + b; b = t - b; }
+template <typename C> __device__ __forceinline__ void bf_mi(C &a, C &b) {          // z = -i
+  const C t = a, v = b;
+  a.x = t.x + v.y; a.y = t.y - v.x;
+  b.x = t.x - v.y; b.y = t.y + v.x;
+}
+// z = exp(-i pi/4) (Q = 0) or -i times it (Q = 1)
+template <int Q, typename C> __device__ __forceinline__ void bf_8th(C &a, C &b) {
+  typedef decltype(a.x) T;
+  const T h = (T) 0.70710678118654752440;
+  const C t = a;
+  const T s = b.x + b.y, d = b.y - b.x;
+  if (Q == 0) {            // z b = h (b.x + b.y, b.y - b.x)
+    a.x = fma_t(h, s, t.x); a.y = fma_t(h, d, t.y);
+    b.x = fma_t(-h, s, t.x); b.y = fma_t(-h, d, t.y);
+  } else {                 // -i z b = h (b.y - b.x, -(b.x + b.y))
+    a.x = fma_t(h, d, t.x); a.y = fma_t(-h, s, t.y);
+    b.x = fma_t(-h, d, t.x); b.y = fma_t(h, s, t.y);
+  }
+}
+
+// level tables of a twiddled butterfly: z2; z4; z8[0..1]; z16[0..3]
+template <int R, typename C> struct PolyTw {
+  C z[R == 2 ? 1 : R == 4 ? 2 : R == 8 ? 4 : 8];
+};
+
+// x[q S], q < M, in place of a register array u; result order j in y[0..M-1]
+template <int M, int S, bool TW, int R, typename C>
+__device__ __forceinline__ void poly_eval(const C *u, C *y, const PolyTw<R, C> &w) {
+  if constexpr (M == 1) {
+    y[0] = u[0];
   } else {
-    for (int idx = threadIdx.x; idx < nR * B; idx += blockDim.x) {
-      const int l = idx % B, i = idx / B;
-      butterfly(l, i, i % p, 1);
+    C e[M / 2], o[M / 2];
+    poly_eval<M / 2, 2 * S, TW, R, C>(u, e, w);
+    poly_eval<M / 2, 2 * S, TW, R, C>(u + S, o, w);
+#pragma unroll
+    for (int j = 0; j < M / 2; j++) {
+      if constexpr (TW) {
+        constexpr int off = M == 2 ? 0 : M == 4 ? 1 : M == 8 ? 2 : 4, Q = M / 4;
+        if (M == 2 || j < Q) bf_z(e[j], o[j], w.z[off + (M == 2 ? 0 : j)]);
+        else bf_miz(e[j], o[j], w.z[off + j - Q]);
+      } else {
+        if (j == 0) bf_1(e[j], o[j]);
+        else if (4 * j == M) bf_mi(e[j], o[j]);
+        else if (8 * j == M) bf_8th<0>(e[j], o[j]);
+        else if (8 * j == 3 * M) bf_8th<1>(e[j], o[j]);
+        else {             // M = 16, odd j: exp(-2 pi i j / 16)
+          C z;
+          if constexpr (sizeof(e[0].x) == 4) {   // (cos, sin)
+            if (j == 1 || j == 5) { z.x = ff::FF_C1; z.y = -ff::FF_S1; } else { z.x = ff::FF_S1; z.y = -ff::FF_C1; }
+          } else {                               // (cos, tan) of -pi/8 and -3 pi/8: tan(pi/8) = sqrt(2) - 1
+            if (j == 1 || j == 5) { z.x = 0.923879532511286756128; z.y = -0.414213562373095048802; }
+            else { z.x = 0.382683432365089771728; z.y = -2.414213562373095048802; }
+          }
+          if (j < 4) bf_z(e[j], o[j], z); else bf_miz(e[j], o[j], z);
+        }
+      }
+      y[j] = e[j];
+      y[j + M / 2] = o[j];
     }
   }
 }
 
-// Runs all stages; returns the buffer holding the result (a or b).
-template <typename T>
-__device__ __forceinline__ typename cplx_t<T>::type *tile_fft(typename cplx_t<T>::type *a,
-                                                              typename cplx_t<T>::type *b,
-                                                              const FftPlan<T> &pl, int B, int ldb, T s) {
+__host__ __device__ constexpr bool is_pow2(int r) { return (r & (r - 1)) == 0; }
+
+// Forward R-point DFT of u_q w^q, w = exp(-2 pi i kt / n), in natural order;
+// TW = false: w = 1.  tw: the plan's table of 2n (FP64) or n (FP32) entries.
+template <int R, bool TW, typename T>
+__device__ __forceinline__ void stage_dft(typename cplx_t<T>::type (&u)[R], int kt, int n,
+                                          const typename cplx_t<T>::type *__restrict__ tw) {
   typedef typename cplx_t<T>::type C;
-  C *in = a, *out = b;
-  int p = 1;
-  for (int st = 0; st < pl.nst; st++) {
-    const int R = pl.radix[st];
-    // FP64 plans use radices up to 8 only (the larger ones would raise the
-    // kernels' register count, and FP64 occupancy with it, for every length)
-    switch (R) {
-      case 8: stockham_stage<8, T>(in, out, pl.n, B, ldb, p, pl.tw, s); break;
-      case 4: stockham_stage<4, T>(in, out, pl.n, B, ldb, p, pl.tw, s); break;
-      case 2: stockham_stage<2, T>(in, out, pl.n, B, ldb, p, pl.tw, s); break;
-      case 3: stockham_stage<3, T>(in, out, pl.n, B, ldb, p, pl.tw, s); break;
-      case 5: stockham_stage<5, T>(in, out, pl.n, B, ldb, p, pl.tw, s); break;
-      default:
-        if constexpr (sizeof(T) == 4) {
-          switch (R) {
-            case 16: stockham_stage<16, T>(in, out, pl.n, B, ldb, p, pl.tw, s); break;
-            case 6: stockham_stage<6, T>(in, out, pl.n, B, ldb, p, pl.tw, s); break;
-            case 9: stockham_stage<9, T>(in, out, pl.n, B, ldb, p, pl.tw, s); break;
-            case 10: stockham_stage<10, T>(in, out, pl.n, B, ldb, p, pl.tw, s); break;
-            case 12: stockham_stage<12, T>(in, out, pl.n, B, ldb, p, pl.tw, s); break;
-            default: stockham_stage<15, T>(in, out, pl.n, B, ldb, p, pl.tw, s); break;
-          }
-        }
-        break;
+  if constexpr (is_pow2(R)) {
+    PolyTw<R, C> w;
+    if constexpr (TW) {
+      if constexpr (sizeof(T) == 8) tw += n;   // the (cos, tan) half
+      w.z[0] = __ldg(&tw[kt * (R / 2)]);
+      if constexpr (R >= 4) w.z[1] = __ldg(&tw[kt * (R / 4)]);
+      if constexpr (R >= 8) { w.z[2] = __ldg(&tw[kt * (R / 8)]); w.z[3] = __ldg(&tw[kt * (R / 8) + n / 8]); }
+      if constexpr (R >= 16)
+#pragma unroll
+        for (int j = 0; j < 4; j++) w.z[4 + j] = __ldg(&tw[kt + j * (n / 16)]);
     }
-    __syncthreads();
+    C y[R];
+    poly_eval<R, 1, TW, R, C>(u, y, w);
+#pragma unroll
+    for (int q = 0; q < R; q++) u[q] = y[q];
+  } else {
+    if constexpr (TW) {
+#pragma unroll
+      for (int q = 1; q < R; q++) u[q] = cmul(u[q], __ldg(&tw[q * kt]));
+    }
+    small_dft<R, C, T>(u, (T) -1);
+  }
+}
+
+// i / d and i % d for i < 65536 by one multiplication (m = ceil(2^32 / d))
+struct FastDiv {
+  unsigned d, m;
+  __device__ __forceinline__ FastDiv(int d_) : d(d_), m(d_ > 1 ? 0xffffffffu / (unsigned) d_ + 1u : 0u) {}
+  __device__ __forceinline__ void divmod(int i, int &q, int &r) const {
+    q = d > 1 ? (int) __umulhi((unsigned) i, m) : i;
+    r = i - q * (int) d;
+  }
+};
+
+// Tile geometry of the line kernels: nl lines of length n, line l at l * LP,
+// element e at e + e/16 (the odd line pitch and the skew keep line-fast and
+// element-fast accesses off each other's banks).
+struct Tile {
+  int n, B, logB, nl, LP;
+  __host__ __device__ static constexpr int pitch(int n) { return (n + (n >> 4)) | 1; }
+  __device__ __forceinline__ int at(int l, int e) const { return l * LP + e + (e >> 4); }
+};
+
+// One stage over the tile: butterfly i of line l takes rd(l, i + q n/R) and
+// gives wr(l, j + q p), j = (i - k) R + k, k = i mod p.  EF: consecutive
+// threads take consecutive butterflies of a line, else consecutive lines.
+// FIRST: p = 1, no twiddles.
+template <int R, bool FIRST, typename T, class Rd, class Wr>
+__device__ __forceinline__ void tile_stage(const Tile &g, int ef, int p, const typename cplx_t<T>::type *__restrict__ tw,
+                                           const Rd &rd, const Wr &wr) {
+  typedef typename cplx_t<T>::type C;
+  const int nR = g.n / R, twstep = FIRST ? 0 : g.n / (p * R);
+  const FastDiv byn(nR), byp(FIRST ? 1 : p);
+  for (int idx = threadIdx.x; idx < g.B * nR; idx += blockDim.x) {
+    int l, i;
+    if (ef) byn.divmod(idx, l, i);
+    else { l = idx & (g.B - 1); i = idx >> g.logB; }
+    if (l >= g.nl) continue;
+    C u[R];
+#pragma unroll
+    for (int q = 0; q < R; q++) u[q] = rd(l, i + q * nR);
+    int k = 0, quo;
+    if (!FIRST) byp.divmod(i, quo, k);
+    (void) quo;
+    stage_dft<R, !FIRST, T>(u, k * twstep, g.n, tw);
+    const int j = (i - k) * R + k;
+#pragma unroll
+    for (int q = 0; q < R; q++) wr(l, j + q * p, u[q]);
+  }
+}
+template <bool FIRST, typename T, class Rd, class Wr>
+__device__ __forceinline__ void run_stage(int R, const Tile &g, int ef, int p,
+                                          const typename cplx_t<T>::type *__restrict__ tw, const Rd &rd, const Wr &wr) {
+  switch (R) {
+    case 16: tile_stage<16, FIRST, T>(g, ef, p, tw, rd, wr); break;
+    case 8: tile_stage<8, FIRST, T>(g, ef, p, tw, rd, wr); break;
+    case 4: tile_stage<4, FIRST, T>(g, ef, p, tw, rd, wr); break;
+    case 2: tile_stage<2, FIRST, T>(g, ef, p, tw, rd, wr); break;
+    case 3: tile_stage<3, FIRST, T>(g, ef, p, tw, rd, wr); break;
+    case 5: tile_stage<5, FIRST, T>(g, ef, p, tw, rd, wr); break;
+    case 6: tile_stage<6, FIRST, T>(g, ef, p, tw, rd, wr); break;
+    case 9: tile_stage<9, FIRST, T>(g, ef, p, tw, rd, wr); break;
+    case 10: tile_stage<10, FIRST, T>(g, ef, p, tw, rd, wr); break;
+    case 12: tile_stage<12, FIRST, T>(g, ef, p, tw, rd, wr); break;
+    default: tile_stage<15, FIRST, T>(g, ef, p, tw, rd, wr); break;
+  }
+}
+
+// Forward FFT of the tile: first stage from rd (ef0), the others from shared
+// memory, the last one into wr (efl) when DIRECT (two stages or more), else
+// the result stays in shared memory and its buffer is returned.  Writes
+// alternate between b0 (first) and b1.
+template <bool DIRECT, typename T, class Rd, class Wr>
+__device__ __forceinline__ typename cplx_t<T>::type *tile_fft(const FftPlan<T> &pl, const Tile &g, int ef0, int efl,
+                                                              typename cplx_t<T>::type *b0,
+                                                              typename cplx_t<T>::type *b1, const Rd &rd, const Wr &wr) {
+  typedef typename cplx_t<T>::type C;
+  C *in = b0, *out = b1;
+  if (pl.nst == 0) {       // length 1
+    for (int l = threadIdx.x; l < g.nl; l += blockDim.x) b0[g.at(l, 0)] = rd(l, 0);
+  } else {
+    run_stage<true, T>(pl.radix[0], g, ef0, 1, pl.tw, rd, [&](int l, int e, C v) { b0[g.at(l, e)] = v; });
+  }
+  __syncthreads();
+  int p = pl.nst ? pl.radix[0] : 1;
+  for (int st = 1; st < pl.nst; st++) {
+    const int R = pl.radix[st];
+    const bool direct = DIRECT && st == pl.nst - 1;
+    run_stage<false, T>(R, g, direct ? efl : ef0, p, pl.tw, [&](int l, int e) { return in[g.at(l, e)]; },
+                        [&](int l, int e, C v) { if (direct) wr(l, e, v); else out[g.at(l, e)] = v; });
+    if (!direct) __syncthreads();
     p *= R;
     C *t = in; in = out; out = t;
   }
   return in;
 }
 
+template <typename C> __device__ __forceinline__ C swap_ri(C v) { C r; r.x = v.y; r.y = v.x; return r; }
+template <typename C> __device__ __forceinline__ C swap_if(C v, bool s) {
+  C r; r.x = s ? v.y : v.x; r.y = s ? v.x : v.y; return r;
+}
+
 // ------------------------------------------------------------ line pass
 enum { LINE_C2C = 0, LINE_R2C = 1, LINE_C2R = 2 };
 
+constexpr int LINE_BATCH = 8;      // fields of one launch
+
 template <typename T> struct LineArgs {
   FftPlan<T> plan;       // length of the complex FFT actually run
-  int B;                 // lines per CTA (divides nb)
+  int B, logB;           // lines per CTA (a power of two)
   int nb;                // extent of the fast line index b
-  T sign;                // -1 forward, +1 inverse
+  int inverse;           // LINE_C2C: 0 forward, 1 inverse
   const typename cplx_t<T>::type *tw2;  // R2C/C2R: table of length 2n
   int e_fast;            // 1: the load functor's fast address index is the element
   int e_fast_store;      // 1: the store functor's fast address index is the element
 };
 
-// Element pitch of a tile of B lines: padded against bank conflicts between
-// lines; a single line (long lines of 1-D grids) needs no padding.
-__host__ __device__ __forceinline__ int tile_pitch(int B) { return B == 1 ? 1 : B + 1; }
-
-// Visits the (line l, element e) pairs of this thread, e < n: element-fast
-// (each line in turn, elements across the threads) or line-fast (thread t
-// on line t % B, elements t / B + j blockDim.x / B); in batches of U whose
-// fetches are all issued before the first put, so that U global loads per
-// thread are in flight together.
-// Element-fast mapping of the threads over a tile's (line, element) pairs:
-// lines shorter than the CTA take several lines per pass (thread t on line
-// t / n + j lpp, element t % n), so that no thread idles for n < blockDim.
-struct EFastMap {
-  int l0, lstep, e0, estep;
-  __device__ __forceinline__ EFastMap(int n) {
-    const int tid = threadIdx.x, nth = blockDim.x;
-    if (n < nth) {
-      lstep = nth / n;
-      l0 = tid / n;
-      e0 = tid - l0 * n;
-      estep = n;
-      if (l0 >= lstep) l0 = 1 << 30;   // the threads past lstep * n have no pair
-    } else {
-      l0 = 0; lstep = 1; e0 = tid; estep = nth;
-    }
-  }
-};
-
-template <int U, class Fetch, class Put>
-__device__ __forceinline__ void batched_tile(int efast, int n, int B, Fetch fetch, Put put) {
-  typedef decltype(fetch(0, 0)) R;
-  const int tid = threadIdx.x, nth = blockDim.x;
-  if (efast) {
-    const EFastMap m(n);
-    for (int e = m.e0; e < n; e += m.estep)
-      for (int l0 = m.l0; l0 < B; l0 += U * m.lstep) {
-        R r[U];
-#pragma unroll
-        for (int u = 0; u < U; u++)
-          if (l0 + u * m.lstep < B) r[u] = fetch(l0 + u * m.lstep, e);
-#pragma unroll
-        for (int u = 0; u < U; u++)
-          if (l0 + u * m.lstep < B) put(l0 + u * m.lstep, e, r[u]);
-      }
-  } else {
-    const int l = tid % B, est = nth / B;
-    for (int e0 = tid / B; e0 < n; e0 += U * est) {
-      R r[U];
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int e = e0 + u * est;
-        if (e < n) r[u] = fetch(l, e);
-      }
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int e = e0 + u * est;
-        if (e < n) put(l, e, r[u]);
-      }
-    }
-  }
-}
-
-template <typename C> struct CPair { C a, b; };
+// The functors of the fields of one launch (blockIdx.z selects).  Functors
+// with kBatch take up to LINE_BATCH fields, the others one.
+template <class F> __host__ __device__ constexpr auto batch_of(int) -> decltype(F::kBatch, bool()) { return F::kBatch; }
+template <class F> __host__ __device__ constexpr bool batch_of(long) { return false; }
+template <class F, int NB> struct Batch { F f[NB]; };
 
 // Line (a, b) = (blockIdx.y, blockIdx.x * B + l), element e.
 //   LINE_C2C: X = FFT(ld(a,b,e)), st(a,b,e,X[e]) for e < n
 //   LINE_R2C: z = ld(a,b,e) (packed even/odd reals), st(a,b,k,X[k]) for k <= n
 //   LINE_C2R: X[k] = ld(a,b,k) for k <= n, st(a,b,e, (x[2e], x[2e+1]))
-template <typename T, int MODE, class Ld, class St>
-__global__ void __launch_bounds__(FFT_THREADS) line_fft_kernel(const LineArgs<T> args, const Ld ld, const St st) {
+// The first stage's butterflies load straight from global memory and the last
+// one's store straight to it, a line crosses shared memory only between
+// stages (n <= 256: once; the staged form it replaces wrote and read it once
+// more at either end and twice per stage).  Inverse transforms run the
+// forward stages on (im, re).  The R2C / C2R steps take k and n - k together
+// (12 and 10 operations a pair).  The last tile may be partial.
+// FP64 is bound by its issue rate of 2 operations per clock and SM, whatever
+// the occupancy, so what counts is operations per element: 22 at n = 128 with
+// radices 8, 8, 2 and separate twiddle products, 18 as 16, 8 with the
+// products inside the butterflies.
+template <typename T, int MODE, int NB, class Ld, class St>
+__global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 3 : 2)
+    line_fft_kernel(const __grid_constant__ LineArgs<T> args, const __grid_constant__ Batch<Ld, NB> lds,
+                    const __grid_constant__ Batch<St, NB> sts) {
   typedef typename cplx_t<T>::type C;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int n = args.plan.n, B = args.B, ldb = tile_pitch(B);
-  C *buf0 = reinterpret_cast<C *>(smem_raw);
-  C *buf1 = buf0 + n * ldb;
-  const int a = blockIdx.y, b0 = blockIdx.x * B;
-  // element-fast side: each line in turn, elements across the threads;
-  // line-fast side: thread t on line t % B, elements t / B + j (blockDim / B)
-  const int tid = threadIdx.x, nth = blockDim.x, lt = tid % B, et0 = tid / B, est = nth / B;
-  (void) lt; (void) et0; (void) est;
-  // the last tile may be partial (B need not divide nb): its missing lines
-  // are transformed as zeros and not stored
-  const int nb = args.nb;
-  const C zero = mk<T>((T) 0, (T) 0);
+  const Ld &ld = lds.f[NB > 1 ? blockIdx.z : 0];
+  const St &st = sts.f[NB > 1 ? blockIdx.z : 0];
+  const int a = blockIdx.y, b0 = blockIdx.x * args.B, n = args.plan.n;
+  Tile g;
+  g.n = n; g.B = args.B; g.logB = args.logB; g.LP = Tile::pitch(n);
+  g.nl = args.nb - b0 < args.B ? args.nb - b0 : args.B;
+  C *buf0 = reinterpret_cast<C *>(smem_raw), *buf1 = buf0 + args.B * g.LP;
+  const FftPlan<T> &pl = args.plan;
+  auto none = [](int, int, C) {};
 
-  // ---- load
-  if (MODE == LINE_C2R) {
-    // Z[k] = (X[k] + X*[n-k]) + i w^{-k} (X[k] - X*[n-k]),  w = exp(-2 pi i / 2n)
-    batched_tile<sizeof(T) == 4 ? 4 : 1>(args.e_fast, n, B,
-        [&](int l, int k) {
-          if (b0 + l >= nb) return CPair<C>{ zero, zero };
-          return CPair<C>{ ld(a, b0 + l, k), ld(a, b0 + l, n - k) };
-        },
-        [&](int l, int k, CPair<C> x) {
-          C xk = x.a, xm = x.b;
-          if (k == 0) { xk.y = (T) 0; xm.y = (T) 0; }   // DC / Nyquist are real
-          C sum = xk + conjc(xm), dif = xk - conjc(xm);
-          C w = __ldg(&args.tw2[k]);
-          w.y = -w.y;                                    // w^{-k}
-          C t = cmul(dif, w);
-          C z; z.x = sum.x - t.y; z.y = sum.y + t.x;     // sum + i t
-          buf0[k * ldb + l] = z;
-        });
-  } else {
-    batched_tile<sizeof(T) == 4 ? 8 : 1>(args.e_fast, n, B, [&](int l, int e) { return b0 + l < nb ? ld(a, b0 + l, e) : zero; },
-                                         [&](int l, int e, C v) { buf0[e * ldb + l] = v; });
-  }
-  __syncthreads();
-
-  C *res = tile_fft<T>(buf0, buf1, args.plan, B, ldb, args.sign);
-
-  // ---- store
-  if (MODE == LINE_R2C) {
-    // X[k] = (Z[k] + Z*[n-k]) / 2 - (i/2) w^k (Z[k] - Z*[n-k]),  k = 0..n
-    auto one = [&](int k, int l) {
-      C zk = res[(k == n ? 0 : k) * ldb + l];
-      C zm = res[(k == 0 ? 0 : n - k) * ldb + l];
-      C sum = zk + conjc(zm), dif = zk - conjc(zm);
-      C w = __ldg(&args.tw2[k == n ? 0 : k]);
-      if (k == n) { w.x = (T) -1; w.y = (T) 0; }
-      C t = cmul(dif, w);
-      C x; x.x = (T) 0.5 * (sum.x + t.y); x.y = (T) 0.5 * (sum.y - t.x);   // (sum - i t)/2
-      if (b0 + l < nb) st(a, b0 + l, k, x);
-    };
-    if (args.e_fast_store) {
-      const EFastMap m(n + 1);
-      for (int k = m.e0; k <= n; k += m.estep)
-        for (int l = m.l0; l < B; l += m.lstep) one(k, l);
-    } else {
-      for (int k = et0; k <= n; k += est) one(k, lt);
+  if constexpr (MODE == LINE_C2R) {
+    // Z[k] = sum + i w^-k dif, sum, dif = X[k] +- X*[n-k], w = exp(-2 pi i / 2n),
+    // and Z[n-k] = conj(2 sum - Z[k]); stored as (im, re) for the inverse
+    const int np = n / 2 + 1;
+    const FastDiv byp(np);
+    for (int idx = threadIdx.x; idx < np * args.B; idx += blockDim.x) {
+      int l, k;
+      if (args.e_fast) byp.divmod(idx, l, k);
+      else { l = idx & (args.B - 1); k = idx >> args.logB; }
+      if (l >= g.nl) continue;
+      C xk = ld(a, b0 + l, k), xm = ld(a, b0 + l, n - k);
+      if (k == 0) { xk.y = (T) 0; xm.y = (T) 0; }   // DC / Nyquist are real
+      const C w = __ldg(&args.tw2[k]);
+      const T sx = xk.x + xm.x, sy = xk.y - xm.y, dx = xk.x - xm.x, dy = xk.y + xm.y;
+      const T zx = fma_t(dx, w.y, fma_t(-dy, w.x, sx)), zy = fma_t(dx, w.x, fma_t(dy, w.y, sy));
+      buf0[g.at(l, k)] = mk<T>(zy, zx);
+      if (k > 0 && 2 * k != n) buf0[g.at(l, n - k)] = mk<T>(fma_t((T) -2, sy, zy), fma_t((T) 2, sx, -zx));
+    }
+    __syncthreads();
+    auto wr = [&](int l, int e, C v) { st(a, b0 + l, e, swap_ri(v)); };
+    C *r = tile_fft<true, T>(pl, g, args.e_fast, args.e_fast_store, buf1, buf0,
+                             [&](int l, int e) { return buf0[g.at(l, e)]; }, wr);
+    if (pl.nst > 1) return;
+    const FastDiv byn(n);
+    for (int idx = threadIdx.x; idx < n * args.B; idx += blockDim.x) {
+      int l, e;
+      byn.divmod(idx, l, e);
+      if (l < g.nl) wr(l, e, r[g.at(l, e)]);
+    }
+  } else if constexpr (MODE == LINE_R2C) {
+    C *r = tile_fft<false, T>(pl, g, args.e_fast, 0, buf0, buf1, [&](int l, int e) { return ld(a, b0 + l, e); }, none);
+    // X[k] = (sum - i w^k dif) / 2, sum, dif = Z[k] +- Z*[n-k], and
+    // X[n-k] = conj(sum - X[k]), k = 0..n/2
+    const int np = n / 2 + 1;
+    const FastDiv byp(np);
+    for (int idx = threadIdx.x; idx < np * args.B; idx += blockDim.x) {
+      int l, k;
+      if (args.e_fast_store) byp.divmod(idx, l, k);
+      else { l = idx & (args.B - 1); k = idx >> args.logB; }
+      if (l >= g.nl) continue;
+      const C zk = r[g.at(l, k)], zm = r[g.at(l, k == 0 ? 0 : n - k)], w = __ldg(&args.tw2[k]);
+      const T sx = zk.x + zm.x, sy = zk.y - zm.y, dx = zk.x - zm.x, dy = zk.y + zm.y;
+      const T px = fma_t(dx, w.y, fma_t(dy, w.x, sx)), py = fma_t(-dx, w.x, fma_t(dy, w.y, sy));
+      st(a, b0 + l, k, mk<T>((T) 0.5 * px, (T) 0.5 * py));
+      if (2 * k != n) st(a, b0 + l, n - k, mk<T>(fma_t((T) -0.5, px, sx), fma_t((T) 0.5, py, -sy)));
     }
   } else {
-    if (args.e_fast_store) {
-      const EFastMap m(n);
-      for (int e = m.e0; e < n; e += m.estep)
-        for (int l = m.l0; l < B; l += m.lstep)
-          if (b0 + l < nb) st(a, b0 + l, e, res[e * ldb + l]);
-    } else {
-      if (b0 + lt < nb)
-        for (int e = et0; e < n; e += est) st(a, b0 + lt, e, res[e * ldb + lt]);
+    const bool inv = args.inverse;
+    auto rd = [&](int l, int e) { return swap_if(ld(a, b0 + l, e), inv); };
+    auto wr = [&](int l, int e, C v) { st(a, b0 + l, e, swap_if(v, inv)); };
+    C *r = tile_fft<true, T>(pl, g, args.e_fast, args.e_fast_store, buf0, buf1, rd, wr);
+    if (pl.nst > 1) return;
+    const FastDiv byn(n);
+    for (int idx = threadIdx.x; idx < n * args.B; idx += blockDim.x) {
+      int l, e;
+      if (args.e_fast_store) byn.divmod(idx, l, e);
+      else { l = idx & (args.B - 1); e = idx >> args.logB; }
+      if (l < g.nl) wr(l, e, r[g.at(l, e)]);
     }
   }
 }
@@ -456,7 +585,8 @@ template <typename T> struct XOut {
 
 template <typename T> struct XConvArgs {
   FftPlan<T> plan;                 // length nx
-  int B, nx, ny, nkz;              // tile width, grid dims, number of kz planes
+  int B, logB, nx, ny, nkz;        // tile width, grid dims, number of kz planes
+  int acc_buf;                     // some output sums several terms
   int kxh, kyh;                    // octant extents nx/2+1, ny/2+1
   int nin, nout;
   const typename cplx_t<T>::type *src[XC_MAX_IN];
@@ -480,96 +610,97 @@ __device__ __forceinline__ typename cplx_t<T>::type apply_kernel(const XTerm<T> 
   return r;
 }
 
-// grid (ny / B, nkz); one CTA = B consecutive y pencils of one kz plane.
-// One input: its spectrum is computed once into a tile and every output is
-// formed from it (3 tiles).  Several inputs: the outputs one after the other,
-// each summing its terms into an accumulator tile, the input of each term
-// transformed when the term is reached (3 tiles instead of inputs + 2, so a
-// CTA holds more pencils; the transforms are the same in number when each
-// input feeds one output).
+// Shared memory tiles of the generic x passes: the spectrum and a work tile,
+// one more for three stages or more, one for the sum of a multi-term output.
+inline int xconv_bufs(int nst, bool multi) { return 2 + (nst >= 3) + (multi ? 1 : 0); }
+
+// grid (ceil(ny / B), nkz); one CTA = B consecutive y pencils of one kz plane
+// (the last tile may be partial: odd ny).  An input's spectrum is left in
+// shared memory and every output's inverse transform reads it there, times its
+// kernel, in its first stage, and stores from its last stage; an output that
+// sums several terms adds them up in a tile first.
 template <typename T>
-__global__ void __launch_bounds__(FFT_THREADS) xconv_kernel(const XConvArgs<T> A) {
+__global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 3 : 2) xconv_kernel(const __grid_constant__ XConvArgs<T> A) {
   typedef typename cplx_t<T>::type C;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int n = A.plan.n, B = A.B, ldb = tile_pitch(B), tile = n * ldb;   // as choose_tile
-  C *bufs = reinterpret_cast<C *>(smem_raw);
-  const int kz = blockIdx.y, y0 = blockIdx.x * B;
-  const size_t plane = (size_t) A.nx * A.ny;
-  const int l = threadIdx.x % B, e0 = threadIdx.x / B, est = blockDim.x / B;   // thread: one pencil
-  constexpr int LU = sizeof(T) == 4 ? 8 : 1;   // loads in flight per thread (FP32)
-
-  // forward transform of input `in` into tile `tin` (scratch `tsc`); returns the result's tile
-  auto forward = [&](int in, C *tin, C *tsc) -> C * {
-    const C *src = A.src[in] + kz * plane + y0;
-    batched_tile<LU>(0, n, B, [&](int ll, int e) { return src[(size_t) e * A.ny + ll]; },
-                     [&](int ll, int e, C v) { tin[e * ldb + ll] = v; });
-    __syncthreads();
-    return tile_fft<T>(tin, tsc, A.plan, B, ldb, (T) -1);
+  Tile g;
+  const int kz = blockIdx.y, y0 = blockIdx.x * A.B;
+  g.n = A.plan.n; g.B = A.B; g.logB = A.logB; g.LP = Tile::pitch(g.n);
+  g.nl = A.ny - y0 < A.B ? A.ny - y0 : A.B;
+  const int tile = A.B * g.LP, ns = A.plan.nst;
+  C *X = reinterpret_cast<C *>(smem_raw), *W = X + tile, *V = W + (ns >= 3 ? tile : 0), *ACC = V + tile;
+  const size_t off = (size_t) kz * A.nx * A.ny + y0;
+  const bool odd = (ns & 1) || ns == 0;   // the number of stage writes: the forward result ends in X
+  auto none = [](int, int, C) {};
+  int cur = -1;
+  auto forward = [&](int in) {
+    if (in == cur) return;
+    cur = in;
+    const C *src = A.src[in] + off;
+    tile_fft<false, T>(A.plan, g, 0, 0, odd ? X : W, odd ? W : X,
+                       [&](int l, int e) { return src[(size_t) e * A.ny + l]; }, none);
   };
-  // inverse transform of tile `acc` (scratch `tsc`) and the store of output `out`
-  auto emit = [&](const XOut<T> &out, C *acc, C *tsc) {
-    C *r = tile_fft<T>(acc, tsc, A.plan, B, ldb, (T) 1);
-    C *dst = out.dst + kz * plane + y0;
-    if (out.accumulate) {
-      batched_tile<LU>(0, n, B, [&](int ll, int e) { return dst[(size_t) e * A.ny + ll]; },
-                       [&](int ll, int e, C v) { dst[(size_t) e * A.ny + ll] = v + r[e * ldb + ll]; });
-    } else {
-      for (int e = e0; e < n; e += est) dst[(size_t) e * A.ny + l] = r[e * ldb + l];
-    }
-    __syncthreads();
-  };
-
-  if (A.nin == 1) {
-    C *X = bufs, *scr0 = bufs + tile, *scr1 = scr0 + tile;
-    C *r = forward(0, X, scr0);
-    if (r != X) {   // an odd number of stages ends in the scratch tile
-      for (int idx = threadIdx.x; idx < tile; idx += blockDim.x) X[idx] = r[idx];
-      __syncthreads();
-    }
-    for (int o = 0; o < A.nout; o++) {
-      const XOut<T> &out = A.out[o];
-      constexpr int U = sizeof(T) == 4 ? 4 : 1;   // elements per batch (FP32): their kernel values loaded together
-      for (int eb = e0; eb < n; eb += U * est) {
-        C acc[U];
-#pragma unroll
-        for (int u = 0; u < U; u++) acc[u] = mk<T>((T) 0, (T) 0);
-        for (int t = out.t0; t < out.t0 + out.nt; t++) {
-          const XTerm<T> &tm = A.term[t];
-#pragma unroll
-          for (int u = 0; u < U; u++) {
-            const int e = eb + u * est;
-            if (e < n) acc[u] = acc[u] + apply_kernel<T>(tm, X[e * ldb + l], e, y0 + l, kz, A);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-          const int e = eb + u * est;
-          if (e < n) scr0[e * ldb + l] = acc[u];
-        }
+  auto emit = [&](const XOut<T> &out, auto rd) {
+    C *dst = out.dst + off;
+    const bool add = out.accumulate;
+    auto wr = [&](int l, int e, C v) {
+      const size_t i = (size_t) e * A.ny + l;
+      v = swap_ri(v);
+      dst[i] = add ? dst[i] + v : v;
+    };
+    C *r = tile_fft<true, T>(A.plan, g, 0, 0, W, V, [&](int l, int e) { return swap_ri(rd(l, e)); }, wr);
+    if (ns <= 1)
+      for (int idx = threadIdx.x; idx < g.n * g.B; idx += blockDim.x) {
+        const int l = idx & (g.B - 1), e = idx >> g.logB;
+        if (l < g.nl) wr(l, e, r[g.at(l, e)]);
       }
-      __syncthreads();
-      emit(out, scr0, scr1);
-    }
-    return;
-  }
-
-  C *X = bufs, *Y = bufs + tile, *ACC = bufs + 2 * tile;
+    __syncthreads();   // the work tiles are free again
+  };
   for (int o = 0; o < A.nout; o++) {
     const XOut<T> &out = A.out[o];
-    if (out.nt == 0) {   // no term: a zero output (added: no change)
-      for (int e = e0; e < n; e += est) ACC[e * ldb + l] = mk<T>((T) 0, (T) 0);
-      __syncthreads();
+    if (out.nt == 1) {
+      const XTerm<T> &tm = A.term[out.t0];
+      forward(tm.in);
+      emit(out, [&](int l, int e) { return apply_kernel<T>(tm, X[g.at(l, e)], e, y0 + l, kz, A); });
+      continue;
     }
-    for (int t = out.t0; t < out.t0 + out.nt; t++) {
-      const XTerm<T> &tm = A.term[t];
-      const C *r = forward(tm.in, X, Y);
-      for (int e = e0; e < n; e += est) {   // each thread its own elements: no barrier before the sum
-        const C v = apply_kernel<T>(tm, r[e * ldb + l], e, y0 + l, kz, A);
-        ACC[e * ldb + l] = t == out.t0 ? v : ACC[e * ldb + l] + v;
+    for (int t = out.t0; t < out.t0 + out.nt || t == out.t0; t++) {   // no term: a zero output
+      if (out.nt) forward(A.term[t].in);
+      for (int idx = threadIdx.x; idx < g.n * g.B; idx += blockDim.x) {
+        const int l = idx & (g.B - 1), e = idx >> g.logB;
+        if (l >= g.nl) continue;
+        const int i = g.at(l, e);
+        C v = out.nt ? apply_kernel<T>(A.term[t], X[i], e, y0 + l, kz, A) : mk<T>((T) 0, (T) 0);
+        ACC[i] = t == out.t0 ? v : ACC[i] + v;
       }
-      __syncthreads();   // the tiles X / Y are free for the next term's input
+      __syncthreads();   // the spectrum's tile is free for the next term's input
     }
-    emit(out, ACC, X);
+    emit(out, [&](int l, int e) { return ACC[g.at(l, e)]; });
+  }
+}
+
+// nx = 1: the x transforms are the identity
+template <typename T> __global__ void xconv_point_kernel(const __grid_constant__ XConvArgs<T> A) {
+  typedef typename cplx_t<T>::type C;
+  const size_t n = (size_t) A.nkz * A.ny;
+  for (size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t) gridDim.x * blockDim.x) {
+    const int kz = (int) (i / A.ny), y = (int) (i - (size_t) kz * A.ny);
+    C in[XC_MAX_IN];
+#pragma unroll
+    for (int k = 0; k < XC_MAX_IN; k++)
+      if (k < A.nin) in[k] = A.src[k][i];
+    for (int o = 0; o < A.nout; o++) {
+      const XOut<T> &out = A.out[o];
+      C v = mk<T>((T) 0, (T) 0);
+      for (int t = out.t0; t < out.t0 + out.nt; t++) {
+        C x = in[0];
+#pragma unroll
+        for (int k = 1; k < XC_MAX_IN; k++)
+          if (A.term[t].in == k) x = in[k];
+        v = v + apply_kernel<T>(A.term[t], x, 0, y, kz, A);
+      }
+      out.dst[i] = out.accumulate ? out.dst[i] + v : v;
+    }
   }
 }
 
@@ -585,7 +716,7 @@ __global__ void __launch_bounds__(FFT_THREADS) xconv_kernel(const XConvArgs<T> A
 // (cn_m1), and separates the same way: (1 + fx)(1 + fy)(1 + fz).
 template <typename T> struct KinArgs {
   FftPlan<T> plan;
-  int B, nx, ny, nz;
+  int B, logB, nx, ny, nz;
   double2 cdt;          // -i dt / (2 m): factor = exp(cdt |k - k0|^2)
   double inv_n;
   double dkx, dky, dkz; // 2 pi / (n step)
@@ -610,24 +741,21 @@ inline void kin_args(KinArgs<T> &K, int nx, int ny, int nz, double step, double2
   K.cn = 0;
 }
 
-// shared memory of the generic kinetic kernel: two tiles + the factor tables
-inline size_t kin_smem(int n, int B, size_t cplx_bytes) {
-  return 2 * (size_t) n * (B + 1) * cplx_bytes + (size_t) (n + B) * cplx_bytes;
-}
-
 __device__ __forceinline__ double kfreq(int i, int n, double dk) {
   return (double) (i < (n + 1) / 2 ? i : i - n) * dk;
 }
 
 template <typename T>
-__global__ void __launch_bounds__(FFT_THREADS) xkinetic_kernel(const KinArgs<T> A) {
+__global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 3 : 2) xkinetic_kernel(const __grid_constant__ KinArgs<T> A) {
   typedef typename cplx_t<T>::type C;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int n = A.plan.n, B = A.B, ldb = B + 1, tile = n * ldb;
-  C *s0 = reinterpret_cast<C *>(smem_raw), *s1 = s0 + tile, *fx = s1 + tile, *fyz = fx + n;
-  const int kz = blockIdx.y, y0 = blockIdx.x * B;
-  const size_t plane = (size_t) A.nx * A.ny;
-  C *base = A.data + kz * plane + y0;
+  Tile g;
+  const int kz = blockIdx.y, y0 = blockIdx.x * A.B;
+  g.n = A.plan.n; g.B = A.B; g.logB = A.logB; g.LP = Tile::pitch(g.n);
+  g.nl = A.ny - y0 < A.B ? A.ny - y0 : A.B;
+  const int n = g.n, B = g.B, tile = B * g.LP;
+  C *X = reinterpret_cast<C *>(smem_raw), *W = X + tile, *fx = W + tile, *fyz = fx + n;
+  C *base = A.data + (size_t) kz * A.nx * A.ny + y0;
   const C c = mk<T>((T) A.cdt.x, (T) A.cdt.y);
   for (int e = threadIdx.x; e < n; e += blockDim.x) {
     const double k = kfreq(e, A.nx, A.dkx) - A.kx0, q = k * k;
@@ -639,29 +767,43 @@ __global__ void __launch_bounds__(FFT_THREADS) xkinetic_kernel(const KinArgs<T> 
     fyz[l] = A.cn ? cprod1p(cn_m1(c, (T) k, (T) A.h), cn_m1(c, (T) kzv, (T) A.h))
                   : cexpm1(mk<T>((T) (A.cdt.x * q), (T) (A.cdt.y * q)));
   }
-  for (int idx = threadIdx.x; idx < n * B; idx += blockDim.x) {
-    const int l = idx % B, e = idx / B;
-    s0[e * ldb + l] = base[(size_t) e * A.ny + l];
-  }
-  __syncthreads();
-  C *r = tile_fft<T>(s0, s1, A.plan, B, ldb, (T) -1);
-  for (int idx = threadIdx.x; idx < n * B; idx += blockDim.x) {
-    const int l = idx % B, e = idx / B;
-    const C a = r[e * ldb + l];
-    r[e * ldb + l] = mul_1p(mk<T>(a.x * (T) A.inv_n, a.y * (T) A.inv_n), cprod1p(fx[e], fyz[l]));
-  }
-  __syncthreads();
-  C *other = (r == s0) ? s1 : s0;
-  C *r2 = tile_fft<T>(r, other, A.plan, B, ldb, (T) 1);
-  for (int idx = threadIdx.x; idx < n * B; idx += blockDim.x) {
-    const int l = idx % B, e = idx / B;
-    base[(size_t) e * A.ny + l] = r2[e * ldb + l];
-  }
+  const int ns = A.plan.nst;
+  const bool odd = (ns & 1) || ns == 0;
+  auto none = [](int, int, C) {};
+  tile_fft<false, T>(A.plan, g, 0, 0, odd ? X : W, odd ? W : X,
+                     [&](int l, int e) { return base[(size_t) e * A.ny + l]; }, none);   // its barriers cover the tables
+  const T inv_n = (T) A.inv_n;
+  auto factor = [&](int l, int e) {
+    const C v = X[g.at(l, e)];
+    return swap_ri(mul_1p(mk<T>(v.x * inv_n, v.y * inv_n), cprod1p(fx[e], fyz[l])));
+  };
+  auto wr = [&](int l, int e, C v) { base[(size_t) e * A.ny + l] = swap_ri(v); };
+  C *r = tile_fft<true, T>(A.plan, g, 0, 0, W, X, factor, wr);
+  if (ns <= 1)
+    for (int idx = threadIdx.x; idx < n * B; idx += blockDim.x) {
+      const int l = idx & (B - 1), e = idx >> g.logB;
+      if (l < g.nl) wr(l, e, r[g.at(l, e)]);
+    }
 }
 
 // ------------------------------------------------------------ launch helpers
-// partial: B need not divide nb (the kernel skips the missing lines of the last tile)
-int choose_tile(int n, int nb, size_t cplx_bytes, int nbufs, int *B, size_t *smem, bool partial = false);
+// Tile of the generic line kernels for lines of length n (largest radix big), nb
+// adjacent lines in each of na planes: lines per CTA, threads and shared memory.  strided: one
+// side's fast index is the line.
+struct TileShape { int B, logB, threads; size_t smem; };
+template <typename T> inline int max_radix(const FftPlan<T> &p) {
+  int r = 1;
+  for (int i = 0; i < p.nst; i++) r = p.radix[i] > r ? p.radix[i] : r;
+  return r;
+}
+size_t max_smem();   // opt-in shared memory of the device
+int choose_tile(int n, int big, int na, int nb, size_t cplx_bytes, int nbufs, bool strided, size_t table, TileShape *t);
+inline int line_bufs(int mode, int nst) { return mode == LINE_C2C ? (nst >= 3 ? 2 : 1) : 2; }
+
+// One launch of the generic line kernel on a given plan and stream.
+template <typename T, int MODE, int NB, class Ld, class St>
+int launch_generic_lines(const FftPlan<T> &plan, const typename cplx_t<T>::type *tw2, int na, int nb, int nf, T sign,
+                         int ef, int efs, const Batch<Ld, NB> &ld, const Batch<St, NB> &st, cudaStream_t stream);
 
 // "Opt-in shared memory already requested" flag per kernel instantiation.
 // It lives in an anonymous namespace so that every translation unit keeps its
@@ -799,6 +941,32 @@ int launch_kin_pass(int n, int na, int nb, float2 cdt, float dk, float k0, const
   }
 }
 
+template <typename T, int MODE, int NB, class Ld, class St>
+int launch_generic_lines(const FftPlan<T> &plan, const typename cplx_t<T>::type *tw2, int na, int nb, int nf, T sign,
+                         int ef, int efs, const Batch<Ld, NB> &ld, const Batch<St, NB> &st, cudaStream_t stream) {
+  typedef typename cplx_t<T>::type C;
+  LineArgs<T> args;
+  args.plan = plan;
+  args.nb = nb;
+  args.inverse = sign > (T) 0;
+  args.tw2 = tw2;
+  args.e_fast = ef;
+  args.e_fast_store = efs;
+  TileShape t;
+  DFT_TRY(choose_tile(plan.n, max_radix(plan), na * nf, nb, sizeof(C), line_bufs(MODE, plan.nst), !ef || !efs, 0, &t));
+  args.B = t.B;
+  args.logB = t.logB;
+  auto kfn = line_fft_kernel<T, MODE, NB, Ld, St>;
+  typedef SmemOptIn<LineArgs<T> (*)(Ld *, St *, int (*)[MODE + 1], int (*)[NB])> Flag;
+  if (t.smem > 48 * 1024 && !Flag::done) {
+    DFT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) max_smem()));
+    Flag::done = true;
+  }
+  kfn<<<dim3((nb + t.B - 1) / t.B, na, nf), t.threads, t.smem, stream>>>(args, ld, st);
+  DFT_CHECK_LAUNCH();
+  return DFTGPU_OK;
+}
+
 // extra_bytes: algorithmic bytes read / written by the fused functors beyond
 // the transformed line data itself (e.g. the potential read by a phase load).
 template <typename T, int MODE, int EF, int EFS, class Ld, class St>
@@ -824,39 +992,35 @@ int launch_lines(int n_fft, int na, int nb, T sign, const Ld &ld, const St &st, 
       if (rc >= 0) return rc;
     }
   }
-  LineArgs<T> args;
-  DFT_TRY(get_plan<T>(n_fft, &args.plan));
-  args.sign = sign;
-  args.nb = nb;
-  args.e_fast = EF;
-  args.e_fast_store = EFS;
-  args.tw2 = nullptr;
-  if (MODE != LINE_C2C) {
-    FftPlan<T> p2;
-    DFT_TRY(get_plan<T>(2 * n_fft, &p2));
-    args.tw2 = p2.tw;
-  }
-  int B; size_t smem;
-  DFT_TRY(choose_tile(n_fft, nb, sizeof(C), 2, &B, &smem, true));
-  args.B = B;
-  auto kfn = line_fft_kernel<T, MODE, Ld, St>;
-  typedef SmemOptIn<LineArgs<T> (*)(Ld *, St *, int (*)[MODE + 1])> Flag;
-  if (smem > 48 * 1024 && !Flag::done) {
-    DFT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) rt().max_smem_optin));
-    Flag::done = true;
-  }
-  if (smem > rt().max_smem_optin) {
-    set_error(DFTGPU_ERR_SIZE, "line FFT n=%d needs %zu bytes of shared memory", n_fft, smem);
-    return DFTGPU_ERR_SIZE;
-  }
-  dim3 grid((nb + B - 1) / B, na);
-  kfn<<<grid, FFT_THREADS, smem, rt().stream>>>(args, ld, st);
-  DFT_CHECK_LAUNCH();
-  return DFTGPU_OK;
+  FftPlan<T> p1, p2;
+  DFT_TRY(get_plan<T>(n_fft, &p1, small_pass(n_fft, na, nb)));
+  p2.tw = nullptr;
+  if (MODE != LINE_C2C) DFT_TRY(get_plan<T>(2 * n_fft, &p2));
+  Batch<Ld, 1> bl{ { ld } };
+  Batch<St, 1> bs{ { st } };
+  return launch_generic_lines<T, MODE, 1>(p1, p2.tw, na, nb, 1, sign, EF, EFS, bl, bs, rt().stream);
 }
 
 template <typename T> int launch_xconv(XConvArgs<T> &A);
 template <typename T> int launch_xkinetic(KinArgs<T> &A);
+
+// the generic kinetic pass on A.plan and a given stream
+template <typename T> int launch_generic_xkinetic(KinArgs<T> &A, cudaStream_t stream) {
+  typedef typename cplx_t<T>::type C;
+  TileShape t;
+  DFT_TRY(choose_tile(A.nx, max_radix(A.plan), A.nz, A.ny, sizeof(C), 2, true, (size_t) A.nx * sizeof(C), &t));
+  A.B = t.B;
+  A.logB = t.logB;
+  auto kfn = xkinetic_kernel<T>;
+  typedef SmemOptIn<KinArgs<T> (*)()> Flag;
+  if (!Flag::done) {
+    DFT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) max_smem()));
+    Flag::done = true;
+  }
+  kfn<<<dim3((A.ny + t.B - 1) / t.B, A.nz), t.threads, t.smem, stream>>>(A);
+  DFT_CHECK_LAUNCH();
+  return DFTGPU_OK;
+}
 
 // ------------------------------------------------------------ fused z + y passes
 // The fused z + y plane passes (cluster kernels, fast_fft.cuh) are selected

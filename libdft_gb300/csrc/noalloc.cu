@@ -33,9 +33,9 @@ namespace {
 
 constexpr size_t NOALLOC_SCRATCH_BYTES = (size_t) 32 << 20;   // spectral scratch, 32 MiB
 // the z, y and x twiddle tables one after the other, each starting on a
-// 256-byte boundary: nz + ny + nx complex values plus padding, at most
-// 4096 + 32 + 1 (a 1-D grid) or 3 * 1024 (a 3-D grid) complex doubles
-constexpr size_t NOALLOC_TW_BYTES = (size_t) 128 << 10;
+// 256-byte boundary: plan_table() entries of nz, ny and nx plus padding, at most
+// 2 (4096 + 32 + 1) (a 1-D grid) or 6 * 1024 (a 3-D grid) complex doubles
+constexpr size_t NOALLOC_TW_BYTES = (size_t) 256 << 10;
 constexpr int TW_ALIGN = 32;   // table offsets in complex values (256 bytes in FP64)
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH_BYTES + NOALLOC_TW_BYTES];
@@ -59,18 +59,6 @@ int scratch_address(int device, unsigned char **out) {
   }
   *out = g_scratch_addr[device];
   return DFTGPU_OK;
-}
-
-// radices for a 2^a 3^b 5^c length, largest power-of-two radix first
-bool radices_for(int n, int *radix, int *nst) {
-  int m = n, k = 0;
-  while (m % 8 == 0 && k < FFT_MAX_STAGES) { radix[k++] = 8; m /= 8; }
-  while (m % 4 == 0 && k < FFT_MAX_STAGES) { radix[k++] = 4; m /= 4; }
-  while (m % 2 == 0 && k < FFT_MAX_STAGES) { radix[k++] = 2; m /= 2; }
-  while (m % 3 == 0 && k < FFT_MAX_STAGES) { radix[k++] = 3; m /= 3; }
-  while (m % 5 == 0 && k < FFT_MAX_STAGES) { radix[k++] = 5; m /= 5; }
-  *nst = k;
-  return m == 1;
 }
 
 // tw[t] = exp(-2 pi i t / n), evaluated in FP64 and rounded once.  In FP32
@@ -97,11 +85,12 @@ template <typename T> __global__ void twiddle_kernel(typename cplx_t<T>::type *t
     double s, c;
     sincospi(-2.0 * (double) tt / (double) n, &s, &c);
     round_unit(c, s, tw[t]);
+    if constexpr (sizeof(T) == 8) tw[n + t] = cos_tan(c, s);
   }
 }
 
-template <typename T> int make_plan(int n, typename cplx_t<T>::type *tw, cudaStream_t s, FftPlan<T> *pl) {
-  if (!radices_for(n, pl->radix, &pl->nst)) {
+template <typename T> int make_plan(int n, bool small, typename cplx_t<T>::type *tw, cudaStream_t s, FftPlan<T> *pl) {
+  if (fft_radices(n, sizeof(T) == 8 ? DFTGPU_FP64 : DFTGPU_FP32, small, pl->radix, &pl->nst) != DFTGPU_OK) {
     set_error(DFTGPU_ERR_SIZE, "noalloc: length %d is not of the form 2^a 3^b 5^c", n);
     return DFTGPU_ERR_SIZE;
   }
@@ -135,22 +124,9 @@ template <typename T> struct HalfStepStore {
 template <typename T, int MODE, class Ld, class St>
 int run_lines(const FftPlan<T> &pl, int na, int nb, T sign, int e_fast, int e_fast_store, const Ld &ld, const St &st,
               cudaStream_t s) {
-  typedef typename cplx_t<T>::type C;
-  LineArgs<T> args;
-  args.plan = pl;
-  args.sign = sign;
-  args.nb = nb;
-  args.e_fast = e_fast;
-  args.e_fast_store = e_fast_store;
-  args.tw2 = nullptr;
-  int B; size_t smem;
-  DFT_TRY(choose_tile(pl.n, nb, sizeof(C), 2, &B, &smem));
-  args.B = B;
-  auto kfn = line_fft_kernel<T, MODE, Ld, St>;
-  if (smem > 48 * 1024) DFT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-  kfn<<<dim3(nb / B, na), FFT_THREADS, smem, s>>>(args, ld, st);
-  DFT_CHECK_LAUNCH();
-  return DFTGPU_OK;
+  Batch<Ld, 1> bl{ { ld } };
+  Batch<St, 1> bs{ { st } };
+  return launch_generic_lines<T, MODE, 1>(pl, nullptr, na, nb, 1, sign, e_fast, e_fast_store, bl, bs, s);
 }
 
 template <typename T>
@@ -160,16 +136,17 @@ int propagate_noalloc_t(void *out, const void *in, const void *pot, int nx, int 
   C *spec = (C *) base;
   C *tw = (C *) (base + NOALLOC_SCRATCH_BYTES);
   // tables placed by the lengths they hold (a 1-D grid's z line is up to 4096 long)
-  const size_t oy = (size_t) (nz + TW_ALIGN - 1) / TW_ALIGN * TW_ALIGN;
-  const size_t ox = oy + (size_t) (ny + TW_ALIGN - 1) / TW_ALIGN * TW_ALIGN;
-  if ((ox + nx) * sizeof(C) > NOALLOC_TW_BYTES) {
+  auto padded = [](int n) { return (plan_table<T>(n) + TW_ALIGN - 1) / TW_ALIGN * TW_ALIGN; };
+  const size_t oy = padded(nz), ox = oy + padded(ny);
+  if ((ox + plan_table<T>(nx)) * sizeof(C) > NOALLOC_TW_BYTES) {
     set_error(DFTGPU_ERR_SIZE, "noalloc: twiddle tables for %dx%dx%d exceed %zu bytes", nx, ny, nz, NOALLOC_TW_BYTES);
     return DFTGPU_ERR_SIZE;
   }
+  const bool small = small_pass(nx, ny, nz);
   FftPlan<T> pz, py, px;
-  DFT_TRY(make_plan<T>(nz, tw, s, &pz));
-  DFT_TRY(make_plan<T>(ny, tw + oy, s, &py));
-  DFT_TRY(make_plan<T>(nx, tw + ox, s, &px));
+  DFT_TRY(make_plan<T>(nz, small, tw, s, &pz));
+  DFT_TRY(make_plan<T>(ny, small, tw + oy, s, &py));
+  DFT_TRY(make_plan<T>(nx, small, tw + ox, s, &px));
   const T hr = (T) (0.5 * dr), hi = (T) (0.5 * di);
   HalfStepLoad<T> ld{(const C *) in, (const C *) pot, ny, nz, hr, hi};
   SpecStoreZ<T> sz{spec, nx, ny};
@@ -179,22 +156,7 @@ int propagate_noalloc_t(void *out, const void *in, const void *pot, int nx, int 
   KinArgs<T> K;
   K.plan = px;
   kin_args<T>(K, nx, ny, nz, step, make_double2(di / (2.0 * mass), -dr / (2.0 * mass)), 0.0, 0.0, 0.0, spec);
-  int B; size_t smem;
-  DFT_TRY(choose_tile(nx, ny, sizeof(C), 2, &B, &smem));
-  smem = kin_smem(nx, B, sizeof(C));
-  K.B = B;
-  int optin = 0, dev = 0;
-  DFT_CUDA(cudaGetDevice(&dev));
-  DFT_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  if (smem > (size_t) optin) {
-    set_error(DFTGPU_ERR_SIZE, "noalloc: kinetic pass for nx=%d needs %zu bytes of shared memory (limit %d)", nx, smem,
-              optin);
-    return DFTGPU_ERR_SIZE;
-  }
-  if (smem > 48 * 1024)
-    DFT_CUDA(cudaFuncSetAttribute(xkinetic_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-  xkinetic_kernel<T><<<dim3(ny / B, nz), FFT_THREADS, smem, s>>>(K);
-  DFT_CHECK_LAUNCH();
+  DFT_TRY(launch_generic_xkinetic<T>(K, s));
   DFT_TRY((run_lines<T, LINE_C2C>(py, nz, nx, (T) 1, 1, 1, ioy, ioy, s)));
   SpecLoadZ<T> lz{spec, nx, ny};
   HalfStepStore<T> st{(C *) out, (const C *) pot, ny, nz, hr, hi};
