@@ -29,6 +29,14 @@
 #include "common.cuh"
 
 namespace dftgpu {
+
+// The functors of the fields of one launch (blockIdx.z selects).  Functors
+// with kBatch take up to LINE_BATCH fields, the others one.
+constexpr int LINE_BATCH = 8;
+template <class F> __host__ __device__ constexpr auto batch_of(int) -> decltype(F::kBatch, bool()) { return F::kBatch; }
+template <class F> __host__ __device__ constexpr bool batch_of(long) { return false; }
+template <class F, int NB> struct Batch { F f[NB]; };
+
 namespace ff {
 
 typedef float2 C;
@@ -345,13 +353,13 @@ template <class F> __host__ __device__ constexpr auto bounded_store_of(int) -> d
 template <class F> __host__ __device__ constexpr bool bounded_store_of(long) { return false; }
 template <class F> __host__ __device__ constexpr auto ahead_of(int) -> decltype(F::kAhead, bool()) { return F::kAhead; }
 template <class F> __host__ __device__ constexpr bool ahead_of(long) { return false; }
-template <int N, int MODE, int B, class Ld> __device__ __forceinline__ void prefetch_ahead(const Ld &ld, int ahead) {
+template <int N, int MODE, int B, int NB, class Ld>
+__device__ __forceinline__ void prefetch_ahead(const Batch<Ld, NB> &lds, int ahead) {
   if constexpr (ahead_of<Ld>(0)) {
-    const int id = blockIdx.y * gridDim.x + blockIdx.x + ahead;
-    if (ahead > 0 && id < (int) (gridDim.x * gridDim.y)) {
-      const int a2 = id / gridDim.x, b2 = (id - a2 * gridDim.x) * B;
-      ld.prefetch_lines(a2, b2, B, MODE == 2 ? N + 1 : N);
-    }
+    const unsigned id = (NB > 1 ? blockIdx.z * gridDim.y + blockIdx.y : blockIdx.y) * gridDim.x + blockIdx.x + ahead;
+    const unsigned row = id / gridDim.x, z = NB > 1 ? row / gridDim.y : 0;
+    if (ahead > 0 && (NB > 1 ? z < gridDim.z : row < gridDim.y))
+      lds.f[z].prefetch_lines(row - z * gridDim.y, (id - row * gridDim.x) * B, B, MODE == 2 ? N + 1 : N);
   }
 }
 
@@ -382,9 +390,13 @@ template <int N, int MODE, int TMA> struct LineSmem {
 // line-fast cooperative loop (used for the transposed side of z passes).
 // TMA: the staged side moves by TMA instead (tensor maps in tm, bounded wait
 // recorded in *fault; a thread whose wait gave up skips its global stores).
-template <int N, int MODE, int MAP, int LDS, int STS, int TMA, class Ld, class St>
+template <int N, int MODE, int MAP, int LDS, int STS, int TMA, int NB, class Ld, class St>
 __device__ __forceinline__ void line_body(const C *__restrict__ tw, const C *__restrict__ tw2, float sign,
-                                          const Ld &ld, const St &st, int ahead, const TmaMaps *tm, int *fault) {
+                                          const Batch<Ld, NB> &lds, const Batch<St, NB> &sts, int ahead,
+                                          const TmaMaps *tm, int *fault) {
+  const Ld &ld = lds.f[NB > 1 ? blockIdx.z : 0];
+  const St &st = sts.f[NB > 1 ? blockIdx.z : 0];
+  if (TMA && NB > 1) tm += blockIdx.z;
   constexpr int E = Shape<N>::E, TL = Shape<N>::TL, B = Shape<N>::B, LP = Shape<N>::LP;
   typedef TmaTile<N, MODE> TT;
   static_assert(!TMA || TT::OK, "TMA tile");
@@ -402,13 +414,13 @@ __device__ __forceinline__ void line_body(const C *__restrict__ tw, const C *__r
     typename Ld::Raw raw[E];
 #pragma unroll
     for (int q = 0; q < E; q++) raw[q] = ld.fetch(a, b0 + l, t + TL * q);
-    prefetch_ahead<N, MODE, B>(ld, ahead);   // after the own loads: issued before it, they are not delayed
+    prefetch_ahead<N, MODE, B, NB>(lds, ahead);   // after the own loads: issued before it, they are not delayed
 #pragma unroll
     for (int q = 0; q < E; q++) v[q] = ld.cook(raw[q]);
   } else if constexpr (LDS == 0) {
 #pragma unroll
     for (int q = 0; q < E; q++) v[q] = ld(a, b0 + l, t + TL * q);
-    prefetch_ahead<N, MODE, B>(ld, ahead);
+    prefetch_ahead<N, MODE, B, NB>(lds, ahead);
   } else {
     if constexpr (TMA) {
       // the tile's boxes by TMA (one thread), completion on an mbarrier
@@ -424,7 +436,7 @@ __device__ __forceinline__ void line_body(const C *__restrict__ tw, const C *__r
         for (int h = 0; h < TT::NBOX; h++) tma_load_3d(sb + h * TT::BOXB, &tm->load, b0 + 16 * h, a, 0, mb);
       }
       ok = mbar_wait(mb, 0, fault);
-      prefetch_ahead<N, MODE, B>(ld, ahead);
+      prefetch_ahead<N, MODE, B, NB>(lds, ahead);
     } else {
       // line-fast cooperative load of the whole tile (C2R: also the Nyquist
       // element N, which lands in the pitch's spare slot), fully unrolled so
@@ -438,7 +450,7 @@ __device__ __forceinline__ void line_body(const C *__restrict__ tw, const C *__r
           sm[sidx(ll, e, LP)] = ld(a, b0 + ll, e);
         }
       }
-      prefetch_ahead<N, MODE, B>(ld, ahead);
+      prefetch_ahead<N, MODE, B, NB>(lds, ahead);
       __syncthreads();
     }
     // element e of this thread's line from the staged tile
@@ -549,36 +561,36 @@ __device__ __forceinline__ void line_body(const C *__restrict__ tw, const C *__r
   }
 }
 
-template <int N, int MODE, int MAP, int LDS, int STS, int TMA, class Ld, class St>
+template <int N, int MODE, int MAP, int LDS, int STS, int TMA, int NB, class Ld, class St>
 __global__ void __launch_bounds__(256) line_kernel(const C *__restrict__ tw, const C *__restrict__ tw2, float sign,
-                                                   const Ld ld, const St st, int ahead,
-                                                   const __grid_constant__ TmaMaps tm, int *fault) {
-  line_body<N, MODE, MAP, LDS, STS, TMA>(tw, tw2, sign, ld, st, ahead, &tm, fault);
+    const __grid_constant__ Batch<Ld, NB> lds, const __grid_constant__ Batch<St, NB> sts, int ahead,
+    const __grid_constant__ Batch<TmaMaps, TMA ? NB : 1> tm, int *fault) {
+  line_body<N, MODE, MAP, LDS, STS, TMA, NB>(tw, tw2, sign, lds, sts, ahead, tm.f, fault);
 }
 // Passes whose store functor asks for it (kBoundedStore: the inverse phase
 // pass, whose operand loads follow the transform): bounded to 48 registers,
 // 5 CTAs per SM, to hide their latency.
-template <int N, int MODE, int MAP, int LDS, int STS, int TMA, class Ld, class St>
-__global__ void __launch_bounds__(256, 5) line_kernel_stsplit(const C *__restrict__ tw, const C *__restrict__ tw2,
-                                                              float sign, const Ld ld, const St st, int ahead,
-                                                              const __grid_constant__ TmaMaps tm, int *fault) {
-  line_body<N, MODE, MAP, LDS, STS, TMA>(tw, tw2, sign, ld, st, ahead, &tm, fault);
+template <int N, int MODE, int MAP, int LDS, int STS, int TMA, int NB, class Ld, class St>
+__global__ void __launch_bounds__(256, 5) line_kernel_stsplit(const C *__restrict__ tw, const C *__restrict__ tw2, float sign,
+    const __grid_constant__ Batch<Ld, NB> lds, const __grid_constant__ Batch<St, NB> sts, int ahead,
+    const __grid_constant__ Batch<TmaMaps, TMA ? NB : 1> tm, int *fault) {
+  line_body<N, MODE, MAP, LDS, STS, TMA, NB>(tw, tw2, sign, lds, sts, ahead, tm.f, fault);
 }
 // Split loads hold all of a thread's operands (two complex per element) at
 // once; the bound keeps them to 80 registers, 3 CTAs per SM, without spills.
-template <int N, int MODE, int MAP, int LDS, int STS, int TMA, class Ld, class St>
-__global__ void __launch_bounds__(256, 3) line_kernel_split(const C *__restrict__ tw, const C *__restrict__ tw2,
-                                                            float sign, const Ld ld, const St st, int ahead,
-                                                            const __grid_constant__ TmaMaps tm, int *fault) {
-  line_body<N, MODE, MAP, LDS, STS, TMA>(tw, tw2, sign, ld, st, ahead, &tm, fault);
+template <int N, int MODE, int MAP, int LDS, int STS, int TMA, int NB, class Ld, class St>
+__global__ void __launch_bounds__(256, 3) line_kernel_split(const C *__restrict__ tw, const C *__restrict__ tw2, float sign,
+    const __grid_constant__ Batch<Ld, NB> lds, const __grid_constant__ Batch<St, NB> sts, int ahead,
+    const __grid_constant__ Batch<TmaMaps, TMA ? NB : 1> tm, int *fault) {
+  line_body<N, MODE, MAP, LDS, STS, TMA, NB>(tw, tw2, sign, lds, sts, ahead, tm.f, fault);
 }
 
 // --------------------------------------------------------------- x pencils
 // LFAST pencils of the spectral layout [kz][x][y]: line (kz, y), element x.
 struct XArgsF {
   int nx, ny, kxh, kyh;
-  int nin, nout, nslice, pad_;
-  const C *src[4];
+  int nin, nout, nslice, split;   // split: blockIdx.z selects the output (each of one term, MODE 0)
+  const C *src[8];
   C *dst[8];
   int acc_out[8];             // 1: dst += result
   int nterm[8], t0[8];        // terms of each output
@@ -663,8 +675,12 @@ __global__ void __launch_bounds__(256, MODE == 1 ? 1 : (MODE == 0 ? 3 : 2)) xcon
   const int half = A.ny / 2;
   const int iylo = y0 < half ? y0 : A.ny - (y0 + B - 1);
   const int iyo = (y <= half ? y : A.ny - y) - iylo;
-  for (int idx = threadIdx.x; idx < A.nslice * KXH * B; idx += 256) {
-    const int s = idx / (KXH * B), r = idx % (KXH * B), ix = r / B, c = r % B;
+  const bool split = MODE == 0 && A.split;
+  const int o0 = split ? blockIdx.z : 0, o1 = split ? o0 + 1 : A.nout;
+  const int own = split ? A.slot[A.t0[o0]] : 0, slot0 = own > 0 ? own : 0;   // a split launch fetches its own kernel slice only
+  const int nload = split ? own >= 0 : A.nslice;
+  for (int idx = threadIdx.x; idx < nload * KXH * B; idx += 256) {
+    const int s = slot0 + idx / (KXH * B), r = idx % (KXH * B), ix = r / B, c = r % B;
     cp_async4(&ks[idx], A.slice_src[s] + ((size_t) kz * A.kxh + ix) * A.kyh + iylo + c);
   }
   cp_async_commit();
@@ -717,21 +733,23 @@ __global__ void __launch_bounds__(256, MODE == 1 ? 1 : (MODE == 0 ? 3 : 2)) xcon
     for (int j = 0; j < E; j++) acc[j] = make_float2(0.f, 0.f);
   }
   __syncthreads();   // sA ready
-  for (int in = 0; in < sA.nin; in++) {
+  ks -= slot0 * KXH * B;
+  const int in0 = split ? sA.in[sA.t0[o0]] : 0, in1 = split ? in0 + 1 : sA.nin;
+  for (int in = in0; in < in1; in++) {
     const C *src = sA.src[in] + kz * plane + y;
     C v[E];
 #pragma unroll
     for (int q = 0; q < E; q++) v[q] = src[(size_t) (t + TL * q) * A.ny];
-    if (in + 1 < sA.nin) {   // the next input's pencils of this CTA into L2 (as MODE 2)
+    if (in + 1 < in1) {   // the next input's pencils of this CTA into L2 (as MODE 2)
       const C *nsrc = sA.src[in + 1] + kz * plane + y0;
       for (int x = threadIdx.x; x < N; x += 256) prefetch_bulk_l2(nsrc + (size_t) x * A.ny, B * sizeof(C));
     }
     transform<N>(v, t, l, -1.f, tw, sm);
-    if (in == 0) {
+    if (in == in0) {
       cp_async_wait_all();
       __syncthreads();   // kernel slices visible to all threads
     }
-    for (int o = 0; o < sA.nout; o++) {
+    for (int o = o0; o < o1; o++) {
       if constexpr (MULTI) {
         if (o == multi) {
           for (int tm = sA.t0[o]; tm < sA.t0[o] + sA.nterm[o]; tm++) {
@@ -824,7 +842,9 @@ __global__ void __launch_bounds__(256) xkinetic_kernel(const C *__restrict__ tw,
 // x pass.  Bounds: MINB CTAs per SM (split load / bounded store variants).
 template <int N, int MAP, int MINB, class Ld, class St>
 __global__ void __launch_bounds__(256, MINB) line_kin_kernel(const C *__restrict__ tw, float2 cdt, float inv_n, float dk,
-                                                             float k0, const Ld ld, const St st, int ahead) {
+                                                             float k0, const __grid_constant__ Batch<Ld, 1> lds,
+                                                             const St st, int ahead) {
+  const Ld &ld = lds.f[0];
   constexpr int E = Shape<N>::E, TL = Shape<N>::TL, B = Shape<N>::B, LP = Shape<N>::LP;
   __shared__ C sm[B * LP];
   __shared__ C fk[N];   // exp(cdt (k - k0)^2) - 1
@@ -836,13 +856,13 @@ __global__ void __launch_bounds__(256, MINB) line_kin_kernel(const C *__restrict
     typename Ld::Raw raw[E];
 #pragma unroll
     for (int q = 0; q < E; q++) raw[q] = ld.fetch(a, b0 + l, t + TL * q);
-    prefetch_ahead<N, 0, B>(ld, ahead);
+    prefetch_ahead<N, 0, B, 1>(lds, ahead);
 #pragma unroll
     for (int q = 0; q < E; q++) v[q] = ld.cook(raw[q]);
   } else {
 #pragma unroll
     for (int q = 0; q < E; q++) v[q] = ld(a, b0 + l, t + TL * q);
-    prefetch_ahead<N, 0, B>(ld, ahead);
+    prefetch_ahead<N, 0, B, 1>(lds, ahead);
   }
   for (int e = threadIdx.x; e < N; e += 256) {
     const float k = (float) (e < (N + 1) / 2 ? e : e - N) * dk - k0;

@@ -170,6 +170,7 @@ size_t max_smem() {
 // of the SM's pipe whatever the number of its active lanes).
 int choose_tile(int n, int big, int na, int nb, size_t cplx_bytes, int nbufs, bool strided, size_t table, TileShape *t) {
   const size_t hard = max_smem();
+
   const int most = cplx_bytes == 16 ? 2560 : 5120;
   int least = strided ? (int) (64 / cplx_bytes) : 1;
   while (cplx_bytes == 16 && least < 32 && least * n < 32 * big) least *= 2;   // a full warp of the largest butterflies
@@ -301,7 +302,7 @@ double xconv_bytes(const XConvArgs<float> &A, int kxh, int kyh) {
 
 template <int N> int fast_xconv(const XConvArgs<float> &A) {
   constexpr int B = ff::Shape<N>::B;
-  if (A.ny % B || (A.ny / 2) % B || A.nin > 4 || A.nout > 8) return -1;
+  if (A.ny % B || (A.ny / 2) % B || A.nin > 8 || A.nout > 8) return -1;
   ff::XArgsF F;
   memset(&F, 0, sizeof(F));
   F.nx = A.nx; F.ny = A.ny; F.kxh = A.nx / 2 + 1; F.kyh = A.ny / 2 + 1;
@@ -336,7 +337,8 @@ template <int N> int fast_xconv(const XConvArgs<float> &A) {
   }
   FftPlan<float> p;
   DFT_TRY(get_plan<float>(N, &p));
-  const int smem = ff::xconv_smem<N>(F.nslice);
+  F.split = A.split;
+  const int smem = ff::xconv_smem<N>(F.split ? 1 : F.nslice);
   // request exactly the dynamic shared memory this launch needs (the kernel
   // also has static shared memory, so the opt-in maximum itself is not valid)
   // MODE 2: one output summing every term; 1: mixed with one multi-term output; 0: single-term outputs
@@ -349,7 +351,7 @@ template <int N> int fast_xconv(const XConvArgs<float> &A) {
     granted[mode] = smem;
   }
   ProfScope prof("fft_x_conv", xconv_bytes(A, F.kxh, F.kyh));
-  const dim3 grid(A.ny / B, A.nkz);
+  const dim3 grid(A.ny / B, A.nkz, F.split ? A.nout : 1);
   if (mode == 2) ff::xconv_kernel<N, 2><<<grid, 256, smem, rt().stream>>>(p.tw, F, multi);
   else if (mode == 1) ff::xconv_kernel<N, 1><<<grid, 256, smem, rt().stream>>>(p.tw, F, multi);
   else ff::xconv_kernel<N, 0><<<grid, 256, smem, rt().stream>>>(p.tw, F, multi);
@@ -375,6 +377,13 @@ template <int N> int fast_xkinetic(const KinArgs<float> &A) {
 
 template <typename T> int launch_xconv(XConvArgs<T> &A) {
   typedef typename cplx_t<T>::type C;
+  // outputs of one term and one input each are independent: one CTA each, but
+  // in FP32 only while the inputs fit into L2 together (above that a CTA that
+  // takes the inputs one after the other, the next one prefetched, is 1 % of
+  // the 256^3 potential faster)
+  A.split = A.nout > 1 && A.nin == A.nout &&
+            (sizeof(T) == 8 || (double) A.nin * A.nkz * A.nx * A.ny * sizeof(C) <= kBatchBytes);
+  for (int o = 0; o < A.nout; o++) A.split &= A.out[o].nt == 1 && A.term[A.out[o].t0].in == o;
   if constexpr (std::is_same<T, float>::value) {
     if (!generic_fft_only()) {
       int rc = -1;
@@ -418,7 +427,7 @@ template <typename T> int launch_xconv(XConvArgs<T> &A) {
     return DFTGPU_OK;
   }
   TileShape t;
-  DFT_TRY(choose_tile(A.nx, max_radix(A.plan), A.nkz, A.ny, sizeof(C), xconv_bufs(A.plan.nst, A.acc_buf), true, 0, &t));
+  DFT_TRY(choose_tile(A.nx, max_radix(A.plan), A.split ? A.nkz * A.nout : A.nkz, A.ny, sizeof(C), xconv_bufs(A.plan.nst, A.acc_buf), true, 0, &t));
   A.B = t.B;
   A.logB = t.logB;
   static bool attr = false;
@@ -426,7 +435,7 @@ template <typename T> int launch_xconv(XConvArgs<T> &A) {
     DFT_CUDA(cudaFuncSetAttribute(xconv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) max_smem()));
     attr = true;
   }
-  xconv_kernel<T><<<dim3((A.ny + t.B - 1) / t.B, A.nkz), t.threads, t.smem, rt().stream>>>(A);
+  xconv_kernel<T><<<dim3((A.ny + t.B - 1) / t.B, A.nkz, A.split ? A.nout : 1), t.threads, t.smem, rt().stream>>>(A);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }

@@ -62,7 +62,8 @@ template <typename T> int get_plan(int n, FftPlan<T> *plan, bool small = false);
 // radix 16 take 21.  Measured on full potentials, radices up to 5 against up
 // to 16 (us): 32^3 291 / 365, 64^3 517 / 541, 96 x 90 x 80 1452 / 1493, 128^3
 // (2^20 values a pass) 3259 / 3230, 160 x 150 x 144 7971 / 7295.
-inline bool small_pass(int n, int na, int nb) { return (size_t) n * na * nb <= (size_t) 1 << 19; }
+// A few long lines (1-D grids) are bound by one SM's FP64 pipe instead.
+inline bool small_pass(int n, int na, int nb) { return (size_t) n * na * nb <= (size_t) 1 << 19 && na * nb >= 16; }
 
 // ------------------------------------------------------------ butterflies
 template <typename C, typename T>
@@ -450,8 +451,6 @@ template <typename C> __device__ __forceinline__ C swap_if(C v, bool s) {
 // ------------------------------------------------------------ line pass
 enum { LINE_C2C = 0, LINE_R2C = 1, LINE_C2R = 2 };
 
-constexpr int LINE_BATCH = 8;      // fields of one launch
-
 template <typename T> struct LineArgs {
   FftPlan<T> plan;       // length of the complex FFT actually run
   int B, logB;           // lines per CTA (a power of two)
@@ -461,12 +460,6 @@ template <typename T> struct LineArgs {
   int e_fast;            // 1: the load functor's fast address index is the element
   int e_fast_store;      // 1: the store functor's fast address index is the element
 };
-
-// The functors of the fields of one launch (blockIdx.z selects).  Functors
-// with kBatch take up to LINE_BATCH fields, the others one.
-template <class F> __host__ __device__ constexpr auto batch_of(int) -> decltype(F::kBatch, bool()) { return F::kBatch; }
-template <class F> __host__ __device__ constexpr bool batch_of(long) { return false; }
-template <class F, int NB> struct Batch { F f[NB]; };
 
 // Line (a, b) = (blockIdx.y, blockIdx.x * B + l), element e.
 //   LINE_C2C: X = FFT(ld(a,b,e)), st(a,b,e,X[e]) for e < n
@@ -566,7 +559,7 @@ __global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 3 : 2)
 // centring phase (-1)^(kx+ky+kz) and the convolution normalisation step^3/N.
 enum { KER_EVEN = 0, KER_ODD_X = 1, KER_ODD_Y = 2, KER_ODD_Z = 3, KER_UNIT = 4 };
 
-constexpr int XC_MAX_IN = 4;
+constexpr int XC_MAX_IN = 8;
 constexpr int XC_MAX_OUT = 8;
 constexpr int XC_MAX_TERMS = 16;
 
@@ -587,6 +580,7 @@ template <typename T> struct XConvArgs {
   FftPlan<T> plan;                 // length nx
   int B, logB, nx, ny, nkz;        // tile width, grid dims, number of kz planes
   int acc_buf;                     // some output sums several terms
+  int split;                       // blockIdx.z selects the output (each of one term)
   int kxh, kyh;                    // octant extents nx/2+1, ny/2+1
   int nin, nout;
   const typename cplx_t<T>::type *src[XC_MAX_IN];
@@ -656,7 +650,7 @@ __global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 3 : 2) xconv_ker
       }
     __syncthreads();   // the work tiles are free again
   };
-  for (int o = 0; o < A.nout; o++) {
+  for (int o = A.split ? blockIdx.z : 0; o < (A.split ? (int) blockIdx.z + 1 : A.nout); o++) {
     const XOut<T> &out = A.out[o];
     if (out.nt == 1) {
       const XTerm<T> &tm = A.term[out.t0];
@@ -800,6 +794,8 @@ size_t max_smem();   // opt-in shared memory of the device
 int choose_tile(int n, int big, int na, int nb, size_t cplx_bytes, int nbufs, bool strided, size_t table, TileShape *t);
 inline int line_bufs(int mode, int nst) { return mode == LINE_C2C ? (nst >= 3 ? 2 : 1) : 2; }
 
+constexpr double kBatchBytes = 48e6;   // FP32 spectra of one launch: less than half of L2
+
 // One launch of the generic line kernel on a given plan and stream.
 template <typename T, int MODE, int NB, class Ld, class St>
 int launch_generic_lines(const FftPlan<T> &plan, const typename cplx_t<T>::type *tw2, int na, int nb, int nf, T sign,
@@ -847,27 +843,29 @@ int *async_fault_flag();
 template <class F> __host__ __device__ constexpr auto spec_z_of(int) -> decltype(F::kSpecZ, bool()) { return F::kSpecZ; }
 template <class F> __host__ __device__ constexpr bool spec_z_of(long) { return false; }
 
-template <int N, int MODE, int MAP, int LDS, int STS, int TMA, class Ld, class St>
-void launch_line_kernel(int na, int nb, const float2 *tw, const float2 *tw2, float sign, const Ld &ld, const St &st,
-                        const ff::TmaMaps &tm, int *fault) {
+template <int N, int MODE, int MAP, int LDS, int STS, int TMA, int NB, class Ld, class St>
+void launch_line_kernel(int na, int nb, int nf, const float2 *tw, const float2 *tw2, float sign, const Batch<Ld, NB> &ld,
+                        const Batch<St, NB> &st, const Batch<ff::TmaMaps, TMA ? NB : 1> &tm, int *fault) {
   constexpr int B = ff::Shape<N>::B;
+  const dim3 grid(nb / B, na, nf);
   if constexpr (LDS == 0 && ff::split_of<Ld>(0)) {
-    auto k = ff::line_kernel_split<N, MODE, MAP, LDS, STS, TMA, Ld, St>;
-    k<<<dim3(nb / B, na), 256, 0, rt().stream>>>(tw, tw2, sign, ld, st, resident_ctas(k), tm, fault);
+    auto k = ff::line_kernel_split<N, MODE, MAP, LDS, STS, TMA, NB, Ld, St>;
+    k<<<grid, 256, 0, rt().stream>>>(tw, tw2, sign, ld, st, resident_ctas(k), tm, fault);
   } else if constexpr (STS == 0 && ff::bounded_store_of<St>(0)) {
-    auto k = ff::line_kernel_stsplit<N, MODE, MAP, LDS, STS, TMA, Ld, St>;
-    k<<<dim3(nb / B, na), 256, 0, rt().stream>>>(tw, tw2, sign, ld, st, resident_ctas(k), tm, fault);
+    auto k = ff::line_kernel_stsplit<N, MODE, MAP, LDS, STS, TMA, NB, Ld, St>;
+    k<<<grid, 256, 0, rt().stream>>>(tw, tw2, sign, ld, st, resident_ctas(k), tm, fault);
   } else {
-    auto k = ff::line_kernel<N, MODE, MAP, LDS, STS, TMA, Ld, St>;
-    k<<<dim3(nb / B, na), 256, 0, rt().stream>>>(tw, tw2, sign, ld, st, resident_ctas(k), tm, fault);
+    auto k = ff::line_kernel<N, MODE, MAP, LDS, STS, TMA, NB, Ld, St>;
+    k<<<grid, 256, 0, rt().stream>>>(tw, tw2, sign, ld, st, resident_ctas(k), tm, fault);
   }
 }
 
 // FP32 power-of-two lengths: register-resident kernel.  EF / EFS: the fast
 // address index of the load / store side is the element (1) or the line (0).
-// Returns -1 when the shape does not fit the kernel (caller falls back).
-template <int N, int MODE, int EF, int EFS, class Ld, class St>
-int launch_fast_lines(int na, int nb, float sign, const Ld &ld, const St &st) {
+// nf fields in one launch.  Returns -1 when the shape does not fit the kernel
+// (caller falls back).
+template <int N, int MODE, int EF, int EFS, int NB, class Ld, class St>
+int launch_fast_lines(int na, int nb, int nf, float sign, const Batch<Ld, NB> &ld, const Batch<St, NB> &st) {
   static_assert(MODE != LINE_R2C || (EF == 1 && EFS == 0), "r2c z pass: element-fast load, line-fast store");
   static_assert(MODE != LINE_C2R || (EF == 0 && EFS == 1), "c2r z pass: line-fast load, element-fast store");
   constexpr int MAP = (EF == 0 && EFS == 0) ? ff::MAP_L : ff::MAP_E;
@@ -879,8 +877,6 @@ int launch_fast_lines(int na, int nb, float sign, const Ld &ld, const St &st) {
   DFT_TRY(get_plan<float>(N, &p1));
   p2.tw = nullptr;
   if (MODE != LINE_C2C) DFT_TRY(get_plan<float>(2 * N, &p2));
-  ff::TmaMaps tm;
-  memset(&tm, 0, sizeof(tm));
   // TMA on the spectral side of the z passes: loads of the c2r / c2c passes,
   // stores of the c2c passes.  The r2c passes keep their store loop: with a
   // TMA store the 256^3 step ran at the same rate (235.4 against 236.6 steps/s).
@@ -889,12 +885,16 @@ int launch_fast_lines(int na, int nb, float sign, const Ld &ld, const St &st) {
   if constexpr (TMA_LD || TMA_ST) {
     if (tma_on()) {
       constexpr int ROWS = ff::TmaTile<N, MODE>::ROWS;
+      Batch<ff::TmaMaps, NB> tm;
+      memset(&tm, 0, sizeof(tm));
       int rc = DFTGPU_OK;
-      if constexpr (TMA_LD) rc = encode_spec_map(&tm.load, ld.spec, ld.nx, ld.ny, ROWS);
-      if constexpr (TMA_ST) if (!rc) rc = encode_spec_map(&tm.store, st.spec, st.nx, st.ny, ROWS);
+      for (int i = 0; i < nf && !rc; i++) {
+        if constexpr (TMA_LD) rc = encode_spec_map(&tm.f[i].load, ld.f[i].spec, ld.f[i].nx, ld.f[i].ny, ROWS);
+        if constexpr (TMA_ST) if (!rc) rc = encode_spec_map(&tm.f[i].store, st.f[i].spec, st.f[i].nx, st.f[i].ny, ROWS);
+      }
       int *fault = rc ? nullptr : async_fault_flag();
       if (fault) {
-        launch_line_kernel<N, MODE, MAP, LDS, STS, 1>(na, nb, p1.tw, p2.tw, sign, ld, st, tm, fault);
+        launch_line_kernel<N, MODE, MAP, LDS, STS, 1, NB>(na, nb, nf, p1.tw, p2.tw, sign, ld, st, tm, fault);
         DFT_CHECK_LAUNCH();
         return DFTGPU_OK;
       }
@@ -902,7 +902,9 @@ int launch_fast_lines(int na, int nb, float sign, const Ld &ld, const St &st) {
       g_last_error = 0;   // the encode failure is not the caller's error
     }
   }
-  launch_line_kernel<N, MODE, MAP, LDS, STS, 0>(na, nb, p1.tw, p2.tw, sign, ld, st, tm, nullptr);
+  Batch<ff::TmaMaps, 1> none;
+  memset(&none, 0, sizeof(none));
+  launch_line_kernel<N, MODE, MAP, LDS, STS, 0, NB>(na, nb, nf, p1.tw, p2.tw, sign, ld, st, none, nullptr);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }
@@ -921,7 +923,7 @@ int launch_kin_lines(int na, int nb, float2 cdt, float inv_n, float dk, float k0
   // per SM); strided lines keep a runtime-stride address per element and get
   // 128 (2 CTAs per SM) so that they do not spill
   auto k = ff::line_kin_kernel<N, MAP, (MAP == ff::MAP_E || !ff::bounded_store_of<St>(0)) ? 3 : 2, Ld, St>;
-  k<<<dim3(nb / B, na), 256, 0, rt().stream>>>(p.tw, cdt, inv_n, dk, k0, ld, st, resident_ctas(k));
+  k<<<dim3(nb / B, na), 256, 0, rt().stream>>>(p.tw, cdt, inv_n, dk, k0, Batch<Ld, 1>{ { ld } }, st, resident_ctas(k));
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }
@@ -967,12 +969,14 @@ int launch_generic_lines(const FftPlan<T> &plan, const typename cplx_t<T>::type 
   return DFTGPU_OK;
 }
 
+// Line passes of nf fields (at most NB) of one shape in one launch.
 // extra_bytes: algorithmic bytes read / written by the fused functors beyond
 // the transformed line data itself (e.g. the potential read by a phase load).
-template <typename T, int MODE, int EF, int EFS, class Ld, class St>
-int launch_lines(int n_fft, int na, int nb, T sign, const Ld &ld, const St &st, double extra_bytes = 0.0) {
+template <typename T, int MODE, int EF, int EFS, int NB, class Ld, class St>
+int launch_lines_batch(int n_fft, int na, int nb, int nf, T sign, const Batch<Ld, NB> &ld, const Batch<St, NB> &st,
+                       double extra_bytes = 0.0) {
   typedef typename cplx_t<T>::type C;
-  const double lines = (double) na * nb;
+  const double lines = (double) na * nb * nf;
   const double data = MODE == LINE_C2C ? 2.0 * n_fft : (2.0 * n_fft + 1.0);
   ProfScope prof(MODE == LINE_C2C ? "fft_line_c2c" : (MODE == LINE_R2C ? "fft_line_r2c" : "fft_line_c2r"),
                  lines * data * sizeof(C) + extra_bytes);
@@ -980,25 +984,35 @@ int launch_lines(int n_fft, int na, int nb, T sign, const Ld &ld, const St &st, 
     if (!generic_fft_only()) {
       int rc = -1;
       switch (n_fft) {
-        case 64: rc = launch_fast_lines<64, MODE, EF, EFS>(na, nb, sign, ld, st); break;
-        case 128: rc = launch_fast_lines<128, MODE, EF, EFS>(na, nb, sign, ld, st); break;
-        case 256: rc = launch_fast_lines<256, MODE, EF, EFS>(na, nb, sign, ld, st); break;
-        case 512: rc = launch_fast_lines<512, MODE, EF, EFS>(na, nb, sign, ld, st); break;
-        case 96: rc = launch_fast_lines<96, MODE, EF, EFS>(na, nb, sign, ld, st); break;
-        case 192: rc = launch_fast_lines<192, MODE, EF, EFS>(na, nb, sign, ld, st); break;
-        case 384: rc = launch_fast_lines<384, MODE, EF, EFS>(na, nb, sign, ld, st); break;
+        case 64: rc = launch_fast_lines<64, MODE, EF, EFS, NB>(na, nb, nf, sign, ld, st); break;
+        case 128: rc = launch_fast_lines<128, MODE, EF, EFS, NB>(na, nb, nf, sign, ld, st); break;
+        case 256: rc = launch_fast_lines<256, MODE, EF, EFS, NB>(na, nb, nf, sign, ld, st); break;
+        case 512: rc = launch_fast_lines<512, MODE, EF, EFS, NB>(na, nb, nf, sign, ld, st); break;
+        case 96: rc = launch_fast_lines<96, MODE, EF, EFS, NB>(na, nb, nf, sign, ld, st); break;
+        case 192: rc = launch_fast_lines<192, MODE, EF, EFS, NB>(na, nb, nf, sign, ld, st); break;
+        case 384: rc = launch_fast_lines<384, MODE, EF, EFS, NB>(na, nb, nf, sign, ld, st); break;
         default: break;
       }
       if (rc >= 0) return rc;
     }
   }
   FftPlan<T> p1, p2;
-  DFT_TRY(get_plan<T>(n_fft, &p1, small_pass(n_fft, na, nb)));
+  DFT_TRY(get_plan<T>(n_fft, &p1, small_pass(n_fft, na * nf, nb)));
   p2.tw = nullptr;
   if (MODE != LINE_C2C) DFT_TRY(get_plan<T>(2 * n_fft, &p2));
-  Batch<Ld, 1> bl{ { ld } };
-  Batch<St, 1> bs{ { st } };
-  return launch_generic_lines<T, MODE, 1>(p1, p2.tw, na, nb, 1, sign, EF, EFS, bl, bs, rt().stream);
+  return launch_generic_lines<T, MODE, NB>(p1, p2.tw, na, nb, nf, sign, EF, EFS, ld, st, rt().stream);
+}
+
+template <typename T, int MODE, int EF, int EFS, class Ld, class St>
+int launch_lines(int n_fft, int na, int nb, T sign, const Ld &ld, const St &st, double extra_bytes = 0.0) {
+  constexpr int NB = batch_of<Ld>(0) && batch_of<St>(0) ? LINE_BATCH : 1;   // one instantiation per functor pair
+  Batch<Ld, NB> l;
+  Batch<St, NB> t;
+  memset(&l, 0, sizeof(l));
+  memset(&t, 0, sizeof(t));
+  l.f[0] = ld;
+  t.f[0] = st;
+  return launch_lines_batch<T, MODE, EF, EFS, NB>(n_fft, na, nb, 1, sign, l, t, extra_bytes);
 }
 
 template <typename T> int launch_xconv(XConvArgs<T> &A);

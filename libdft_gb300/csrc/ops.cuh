@@ -14,11 +14,16 @@ template <class F> __global__ void each_kernel(size_t n, F f) {
 // f(0..n-1), independent of one another, spread round-robin over the work
 // stream and the auxiliary streams with event fork / join, so that a CUDA
 // graph captured from the work stream gets them as parallel branches.  Runs
-// on the work stream alone while the profiler is on (per-launch timings).
+// on the work stream alone while the profiler is on (per-launch timings), and
+// on the branch it is in when called from one.
+inline bool &inside_par() {
+  static thread_local bool v = false;
+  return v;
+}
 template <class F> int par_for(int n, F f) {
   cudaStream_t *aux;
   cudaEvent_t *ev;
-  const int ns = prof_on() || n < 2 ? 1 : par_streams(&aux, &ev);
+  const int ns = prof_on() || n < 2 || inside_par() ? 1 : par_streams(&aux, &ev);
   if (ns < 2) {
     for (int i = 0; i < n; i++) DFT_TRY(f(i));
     return DFTGPU_OK;
@@ -28,10 +33,12 @@ template <class F> int par_for(int n, F f) {
   DFT_CUDA(cudaEventRecord(ev[0], main));
   for (int k = 0; k < use - 1; k++) DFT_CUDA(cudaStreamWaitEvent(aux[k], ev[0], 0));
   int rc = DFTGPU_OK;
+  inside_par() = true;
   for (int i = 0; i < n && rc == DFTGPU_OK; i++) {
     rt().stream = i % use == 0 ? main : aux[i % use - 1];
     rc = f(i);
   }
+  inside_par() = false;
   rt().stream = main;
   for (int k = 0; k < use - 1; k++) {
     DFT_CUDA(cudaEventRecord(ev[k + 1], aux[k]));
@@ -52,18 +59,27 @@ template <class F> int launch_each(size_t n, F f, double bytes = 0.0, const char
   return DFTGPU_OK;
 }
 
-// One CTA per (x, y) row of an [nx][ny][nz] grid, threads along z: the
-// lambda gets f(x, y, z, i) with i the linear index, no index division.
+// The (x, y) rows of an [nx][ny][nz] grid, threads along z, a row of more
+// than 256 values in equal segments (blockIdx.z): the lambda gets f(x, y, z, i)
+// with i the linear index, no index division.  Few rows (1-D grids: one) are
+// cut into segments of 32 values, one warp each, so that they use many SMs: a
+// 4096-point row's second OT pass took 150 us on one SM.
+struct RowShape { dim3 grid; int bd; };
+inline RowShape row_shape(int nx, int ny, int nz) {
+  int nseg = (nz + 255) / 256;
+  if ((size_t) nx * ny * nseg < (size_t) 2 * rt().num_sms) nseg = (nz + 31) / 32;
+  const int bd = ((nz + nseg - 1) / nseg + 31) / 32 * 32;
+  return RowShape{ dim3(ny, nx, (nz + bd - 1) / bd), bd };
+}
 template <class F> __global__ void rows_kernel(int ny, int nz, F f) {
-  const int y = blockIdx.x, x = blockIdx.y;
-  const int base = (x * ny + y) * nz;
-  for (int z = threadIdx.x; z < nz; z += blockDim.x) f(x, y, z, base + z);
+  const int y = blockIdx.x, x = blockIdx.y, z = blockIdx.z * blockDim.x + threadIdx.x;
+  if (z < nz) f(x, y, z, (x * ny + y) * nz + z);
 }
 
 template <class F> int launch_rows(int nx, int ny, int nz, F f, double bytes = 0.0, const char *name = "pointwise") {
-  int bd = nz < 256 ? ((nz + 31) / 32) * 32 : 256;
+  const RowShape r = row_shape(nx, ny, nz);
   ProfScope prof(name, bytes);
-  rows_kernel<<<dim3(ny, nx), bd, 0, rt().stream>>>(ny, nz, f);
+  rows_kernel<<<r.grid, r.bd, 0, rt().stream>>>(ny, nz, f);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }
@@ -71,15 +87,14 @@ template <class F> int launch_rows(int nx, int ny, int nz, F f, double bytes = 0
 // The same with a register budget for MINB resident 256-thread CTAs per SM:
 // for latency-bound passes with many independent loads per element.
 template <int MINB, class F> __global__ void __launch_bounds__(256, MINB) rows_kernel_b(int ny, int nz, F f) {
-  const int y = blockIdx.x, x = blockIdx.y;
-  const int base = (x * ny + y) * nz;
-  for (int z = threadIdx.x; z < nz; z += blockDim.x) f(x, y, z, base + z);
+  const int y = blockIdx.x, x = blockIdx.y, z = blockIdx.z * blockDim.x + threadIdx.x;
+  if (z < nz) f(x, y, z, (x * ny + y) * nz + z);
 }
 template <int MINB, class F>
 int launch_rows_b(int nx, int ny, int nz, F f, double bytes = 0.0, const char *name = "pointwise") {
-  int bd = nz < 256 ? ((nz + 31) / 32) * 32 : 256;
+  const RowShape r = row_shape(nx, ny, nz);
   ProfScope prof(name, bytes);
-  rows_kernel_b<MINB><<<dim3(ny, nx), bd, 0, rt().stream>>>(ny, nz, f);
+  rows_kernel_b<MINB><<<r.grid, r.bd, 0, rt().stream>>>(ny, nz, f);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }
@@ -174,6 +189,7 @@ template <int NV, class F> int reduce_host(size_t n, F f, double *out, double sc
 // ---------------------------------------------------------------- functors
 // Spectral layout [kz][x][y]; real / complex grids [x][y][z].
 template <typename T> struct SpecStoreZ {           // z pass output
+  static constexpr bool kBatch = true;
   static constexpr bool kSpecZ = true;
   typename cplx_t<T>::type *spec; int nx, ny;
   __device__ void operator()(int x, int y, int k, typename cplx_t<T>::type v) const {
@@ -184,6 +200,7 @@ template <typename T> struct SpecStoreZ {           // z pass output
 // every thread of a CTA of the line kernels: bring the input of lines
 // (a, b0 .. b0+nl-1), elements 0 .. ne-1, into L2 (bulk prefetches).
 template <typename T> struct SpecLoadZ {            // z pass input (inverse); its tiles are one short
+  static constexpr bool kBatch = true;
   typedef typename cplx_t<T>::type C;                // run per plane, not prefetched ahead
   static constexpr bool kSpecZ = true;
   const C *spec; int nx, ny;
@@ -192,6 +209,7 @@ template <typename T> struct SpecLoadZ {            // z pass input (inverse); i
   }
 };
 template <typename T> struct SpecLineY {            // y pass in place: line (kz, x), element y
+  static constexpr bool kBatch = true;
   typedef typename cplx_t<T>::type C;
   static constexpr bool kAhead = true;
   typename cplx_t<T>::type *spec; int nx, ny;
@@ -206,6 +224,7 @@ template <typename T> struct SpecLineY {            // y pass in place: line (kz
   }
 };
 template <typename T> struct RealPairLoad {         // packed (f[2e], f[2e+1]) of a real row
+  static constexpr bool kBatch = true;
   static constexpr bool kAhead = true;
   const T *f; int ny, nz;
   __device__ void prefetch_lines(int x, int y0, int nl, int) const {      // nl whole rows, contiguous
@@ -218,6 +237,7 @@ template <typename T> struct RealPairLoad {         // packed (f[2e], f[2e+1]) o
   }
 };
 template <typename T> struct RealPairStore {        // real row <- scale * (re, im)
+  static constexpr bool kBatch = true;
   T *f; int ny, nz; T scale;
   __device__ void operator()(int x, int y, int e, typename cplx_t<T>::type v) const {
     T *row = f + ((size_t) x * ny + y) * nz;
@@ -296,10 +316,17 @@ template <typename T> struct CplxLoad {
 int launch_zy_r2c(const RealPairLoad<float> &ld, float2 *spec, int nx, int ny, int nz);
 int launch_yz_c2r(const float2 *spec, const RealPairStore<float> &st, int nx, int ny, int nz);
 
-// y passes over nkz planes of a spectral buffer
+// y passes over nkz planes of nf spectral buffers (ny = 1: the identity)
+template <typename T>
+int ypass_batch(typename cplx_t<T>::type *const *spec, int nf, int nx, int ny, int nkz, T sign) {
+  if (ny == 1) return DFTGPU_OK;
+  Batch<SpecLineY<T>, LINE_BATCH> io;
+  memset(&io, 0, sizeof(io));
+  for (int i = 0; i < nf; i++) io.f[i] = SpecLineY<T>{spec[i], nx, ny};
+  return launch_lines_batch<T, LINE_C2C, 1, 1, LINE_BATCH>(ny, nkz, nx, nf, sign, io, io);
+}
 template <typename T> int ypass(typename cplx_t<T>::type *spec, int nx, int ny, int nkz, T sign) {
-  SpecLineY<T> io{spec, nx, ny};
-  return launch_lines<T, LINE_C2C, 1, 1>(ny, nkz, nx, sign, io, io);
+  return ypass_batch<T>(&spec, 1, nx, ny, nkz, sign);
 }
 
 // forward r2c of a real field through its z and y passes, with a custom
@@ -326,6 +353,60 @@ int irfft_yz(typename cplx_t<T>::type *spec, const St &st, int nx, int ny, int n
   DFT_TRY(ypass<T>(spec, nx, ny, nz / 2 + 1, (T) 1));
   SpecLoadZ<T> ld{spec, nx, ny};
   return launch_lines<T, LINE_C2R, 0, 1>(nz / 2, nx, ny, (T) 1, ld, st, extra_bytes);
+}
+
+// Fields transformed by one launch: all (up to LINE_BATCH) in FP64, whose
+// passes are bound by the FP64 pipe; in FP32 as many as keep the batch's
+// spectra in L2 between their z and y passes (the fused plane passes, when
+// selected, take one).  Full potential, FP32, us: 128^3 (8.5 MB a spectrum) 318
+// one at a time on two branches, 275 five at a time, 286 all eight; 160 x 150 x
+// 144 844 / 838 / 861; 192^3 (28 MB) 925 one at a time, 939 three.  Up to 64^3
+// the step is launch-bound and all go together (64^3 191 / 123).
+template <typename T> inline int batch_fields(int nx, int ny, int nz) {
+  if (sizeof(T) == 8) return LINE_BATCH;
+  if (!fused_zy_off()) return 1;
+  const double spec = 8.0 * (nz / 2 + 1) * nx * ny;
+  const int k = (int) (kBatchBytes / spec);
+  return k < 1 ? 1 : k > LINE_BATCH ? LINE_BATCH : k;
+}
+
+// The z and y passes of nf real fields, batch_fields() at a time, the batches
+// on parallel branches.
+template <typename T>
+int rfft_zy_n(const T *const *f, typename cplx_t<T>::type *const *spec, int nf, int nx, int ny, int nz) {
+  const int k = batch_fields<T>(nx, ny, nz);
+  return par_for((nf + k - 1) / k, [&](int j) -> int {
+    const int i0 = j * k, m = nf - i0 < k ? nf - i0 : k;
+    if (m == 1) return rfft_zy<T>(RealPairLoad<T>{f[i0], ny, nz}, spec[i0], nx, ny, nz);
+    Batch<RealPairLoad<T>, LINE_BATCH> ld;
+    Batch<SpecStoreZ<T>, LINE_BATCH> st;
+    memset(&ld, 0, sizeof(ld));
+    memset(&st, 0, sizeof(st));
+    for (int i = 0; i < m; i++) {
+      ld.f[i] = RealPairLoad<T>{f[i0 + i], ny, nz};
+      st.f[i] = SpecStoreZ<T>{spec[i0 + i], nx, ny};
+    }
+    DFT_TRY((launch_lines_batch<T, LINE_R2C, 1, 0, LINE_BATCH>(nz / 2, nx, ny, m, (T) -1, ld, st)));
+    return ypass_batch<T>(spec + i0, m, nx, ny, nz / 2 + 1, (T) -1);
+  });
+}
+template <typename T>
+int irfft_yz_n(typename cplx_t<T>::type *const *spec, T *const *f, int nf, int nx, int ny, int nz) {
+  const int k = batch_fields<T>(nx, ny, nz);
+  return par_for((nf + k - 1) / k, [&](int j) -> int {
+    const int i0 = j * k, m = nf - i0 < k ? nf - i0 : k;
+    if (m == 1) return irfft_yz<T>(spec[i0], RealPairStore<T>{f[i0], ny, nz, (T) 1}, nx, ny, nz);
+    Batch<SpecLoadZ<T>, LINE_BATCH> ld;
+    Batch<RealPairStore<T>, LINE_BATCH> st;
+    memset(&ld, 0, sizeof(ld));
+    memset(&st, 0, sizeof(st));
+    for (int i = 0; i < m; i++) {
+      ld.f[i] = SpecLoadZ<T>{spec[i0 + i], nx, ny};
+      st.f[i] = RealPairStore<T>{f[i0 + i], ny, nz, (T) 1};
+    }
+    DFT_TRY(ypass_batch<T>(spec + i0, m, nx, ny, nz / 2 + 1, (T) 1));
+    return launch_lines_batch<T, LINE_C2R, 0, 1, LINE_BATCH>(nz / 2, nx, ny, m, (T) 1, ld, st);
+  });
 }
 
 }  // namespace dftgpu

@@ -355,7 +355,7 @@ template <typename T> static int potential_t(dft_ot_functional *otf, cgrid *Pg, 
     if (loc) { sp[n] = s[2]; dst[n++] = r[R_RB]; }
     if (kc) { sp[n] = s[3]; dst[n++] = r[R_RT]; }
     if (bf) { sp[n] = s[7]; dst[n++] = r[R_A]; }
-    DFT_TRY(par_for(n, [&](int i) { return F.inv(sp[i], dst[i]); }));
+    DFT_TRY(F.inv_n(n, sp, dst));
   }
 
   // pointwise 1
@@ -437,32 +437,36 @@ template <typename T> static int potential_t(dft_ot_functional *otf, cgrid *Pg, 
       in[n] = r[R_E]; sp[n++] = s[4];
       for (int a = 0; a < 3; a++) { in[n] = r[R_B0 + a]; sp[n++] = s[5 + a]; }
     }
-    DFT_TRY(par_for(n, [&](int i) { return F.fwd(in[i], sp[i]); }));
+    DFT_TRY(F.fwd_n(n, in, sp));
   }
 
-  // x pass 2: the KC and BF chains are independent
-  auto kc_chain = [&]() -> int {
-    // J_a = F s_a^ in place (src/ot.c:652)
-    XConvArgs<T> B; xc_init(B, P);
-    for (int a = 0; a < 3; a++) xc_in(B, (const C *) s[1 + a]);
-    for (int a = 0; a < 3; a++) { xc_out(B, s[1 + a]); xc_term(B, a, F.k(OT_F), KER_EVEN, (T) 1); }
-    DFT_TRY(launch_xconv<T>(B));
-    for (int a = 0; a < 3; a++) DFT_TRY(F.inv(s[1 + a], r[R_J0 + a]));
-    return DFTGPU_OK;
-  };
-  auto bf_chain = [&]() -> int {   // B_a = V_j (rho v_a)^ in place (+ C = V_j (rho|v|^2)^ when clamped)
-    XConvArgs<T> A; xc_init(A, P);
-    for (int a = 0; a < 3; a++) xc_in(A, (const C *) s[5 + a]);
-    for (int a = 0; a < 3; a++) { xc_out(A, s[5 + a]); xc_term(A, a, F.k(OT_VJ), KER_EVEN, (T) 1); }
-    if (!cmerge) { xc_in(A, (const C *) s[4]); xc_out(A, s[10]); xc_term(A, 3, F.k(OT_VJ), KER_EVEN, (T) 1); }
-    DFT_TRY(launch_xconv<T>(A));
-    if (!cmerge) DFT_TRY(F.inv(s[10], r[R_C]));
-    for (int a = 0; a < 3; a++) DFT_TRY(F.inv(s[5 + a], r[R_BB0 + a]));
-    return DFTGPU_OK;
-  };
-  if (kc && bf) DFT_TRY(par_for(2, [&](int i) { return i == 0 ? kc_chain() : bf_chain(); }));
-  else if (kc) DFT_TRY(kc_chain());
-  else if (bf) DFT_TRY(bf_chain());
+  // x pass 2: J_a = F s_a^ (src/ot.c:652), B_a = V_j (rho v_a)^ and, when
+  // clamped, C = V_j (rho|v|^2)^, all in place.  The convolutions of one launch
+  // and the inverse transforms: all together where they are batched, else a
+  // KC and a BF chain on parallel branches.
+  {
+    C *sp[8]; T *dst[8]; const T *ker[8]; int n = 0, nkc = 0;
+    if (kc) for (int a = 0; a < 3; a++) { sp[n] = s[1 + a]; ker[n] = F.k(OT_F); dst[n++] = r[R_J0 + a]; }
+    nkc = n;
+    if (bf) {
+      for (int a = 0; a < 3; a++) { sp[n] = s[5 + a]; ker[n] = F.k(OT_VJ); dst[n++] = r[R_BB0 + a]; }
+      if (!cmerge) { sp[n] = s[4]; ker[n] = F.k(OT_VJ); dst[n++] = r[R_C]; }
+    }
+    auto chain = [&](int i0, int i1) -> int {
+      XConvArgs<T> A; xc_init(A, P);
+      for (int i = i0; i < i1; i++) xc_in(A, (const C *) sp[i]);
+      for (int i = i0; i < i1; i++) {
+        C *out = sp[i] == s[4] ? s[10] : sp[i];   // (rho|v|^2)^ is kept
+        xc_out(A, out); xc_term(A, i - i0, ker[i], KER_EVEN, (T) 1);
+        sp[i] = out;
+      }
+      DFT_TRY(launch_xconv<T>(A));
+      return F.inv_n(i1 - i0, sp + i0, dst + i0);
+    };
+    if (n > nkc && nkc > 0 && batch_fields<T>(nx, ny, nz) < n)
+      DFT_TRY(par_for(2, [&](int i) { return i == 0 ? chain(0, nkc) : chain(nkc, n); }));
+    else if (n > 0) DFT_TRY(chain(0, n));
+  }
 
   // pointwise 2
   if (kc || bf) {
@@ -646,12 +650,11 @@ template <typename T> static int energy_density_t(dft_ot_functional *otf, rgrid 
     if (kc) { xc_out(A, s[3]); xc_term(A, 0, F.k(OT_F), KER_EVEN, (T) 1); }
     if (bf) { xc_out(A, s[4]); xc_term(A, bfhd ? 1 : 0, F.k(OT_VJ), KER_EVEN, (T) 1); }
     DFT_TRY(launch_xconv<T>(A));
-    if (plain) {
-      DFT_TRY(F.inv(s[1], r[R_U]));
-      DFT_TRY(F.inv(s[2], r[R_RB]));
-    }
-    if (kc) DFT_TRY(F.inv(s[3], r[R_RT]));
-    if (bf) DFT_TRY(F.inv(s[4], r[R_A]));
+    C *sp[4]; T *dst[4]; int n = 0;
+    if (plain) { sp[n] = s[1]; dst[n++] = r[R_U]; sp[n] = s[2]; dst[n++] = r[R_RB]; }
+    if (kc) { sp[n] = s[3]; dst[n++] = r[R_RT]; }
+    if (bf) { sp[n] = s[4]; dst[n++] = r[R_A]; }
+    DFT_TRY(F.inv_n(n, sp, dst));
   }
   {
     const T c2 = (T) otf->c2, c3 = (T) otf->c3, irs = (T) (1.0 / otf->rho_0s), inv2h = (T) (1.0 / (2.0 * P->step));
@@ -697,23 +700,16 @@ template <typename T> static int energy_density_t(dft_ot_functional *otf, rgrid 
       ed[i] = acc;
     }, nb * (4 + (kc ? 5 : 0) + (bf ? 10 : 0)), "ed_pointwise_1"));
   }
-  if (kc) {
-    for (int a = 0; a < 3; a++) DFT_TRY(F.fwd(r[R_S0 + a], s[1 + a]));
+  if (kc || bf) {   // s_a <- F * s_a; rho|v|^2, rho v_a <- V_j * them
+    const T *in[7]; C *sp[7]; T *dst[7]; int n = 0;
     XConvArgs<T> A; xc_init(A, P);
-    for (int a = 0; a < 3; a++) xc_in(A, (const C *) s[1 + a]);
-    for (int a = 0; a < 3; a++) { xc_out(A, s[1 + a]); xc_term(A, a, F.k(OT_F), KER_EVEN, (T) 1); }
+    if (kc) for (int a = 0; a < 3; a++) { in[n] = dst[n] = r[R_S0 + a]; sp[n++] = s[1 + a]; }
+    if (bf) for (int a = 0; a < 4; a++) { in[n] = dst[n] = r[a == 0 ? R_E : R_B0 + a - 1]; sp[n++] = s[4 + a]; }
+    DFT_TRY(F.fwd_n(n, in, sp));
+    for (int i = 0; i < n; i++) xc_in(A, (const C *) sp[i]);
+    for (int i = 0; i < n; i++) { xc_out(A, sp[i]); xc_term(A, i, F.k(kc && i < 3 ? OT_F : OT_VJ), KER_EVEN, (T) 1); }
     DFT_TRY(launch_xconv<T>(A));
-    for (int a = 0; a < 3; a++) DFT_TRY(F.inv(s[1 + a], r[R_S0 + a]));   // s_a <- F * s_a
-  }
-  if (bf) {
-    DFT_TRY(F.fwd(r[R_E], s[4]));
-    for (int a = 0; a < 3; a++) DFT_TRY(F.fwd(r[R_B0 + a], s[5 + a]));
-    XConvArgs<T> A; xc_init(A, P);
-    for (int a = 0; a < 4; a++) xc_in(A, (const C *) s[4 + a]);
-    for (int a = 0; a < 4; a++) { xc_out(A, s[4 + a]); xc_term(A, a, F.k(OT_VJ), KER_EVEN, (T) 1); }
-    DFT_TRY(launch_xconv<T>(A));
-    DFT_TRY(F.inv(s[4], r[R_E]));
-    for (int a = 0; a < 3; a++) DFT_TRY(F.inv(s[5 + a], r[R_B0 + a]));
+    DFT_TRY(F.inv_n(n, sp, dst));
   }
   if (kc || bf) {
     const T f = (T) (-otf->alpha_s / (4.0 * otf->mass)), cm = (T) (otf->c_bfpot * otf->mass);

@@ -39,6 +39,8 @@ template <typename T> struct Fields {
     RealPairLoad<T> ld{f, ny, nz};
     return rfft_zy<T>(ld, spec, nx, ny, nz);
   }
+  int fwd_n(int n, const T *const *f, C *const *spec) { return rfft_zy_n<T>(f, spec, n, nx, ny, nz); }
+  int inv_n(int n, C *const *spec, T *const *f) { return irfft_yz_n<T>(spec, f, n, nx, ny, nz); }
   int inv(C *spec, T *f) {
     RealPairStore<T> st{f, ny, nz, (T) 1};
     return irfft_yz<T>(spec, st, nx, ny, nz);
