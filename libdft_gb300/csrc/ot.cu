@@ -361,6 +361,7 @@ template <typename T> static int potential_t(dft_ot_functional *otf, cgrid *Pg, 
   // pointwise 1
   {
     const T c2 = (T) otf->c2, c3 = (T) otf->c3, irs = (T) (1.0 / otf->rho_0s);
+    const T c2h = c2 / (T) 2, c3t = c3 / (T) 3;   // here, not per point: FP64 divisions cost 10 operations each
     T *rb = r[R_RB], *rt = r[R_RT], *q = r[R_Q];
     T *s0 = r[R_S0], *s1 = r[R_S1], *s2 = r[R_S2];
     T *v0 = r[R_V0], *v1 = r[R_V1], *v2 = r[R_V2], *e = r[R_E], *b0 = r[R_B0], *b1 = r[R_B1], *b2 = r[R_B2];
@@ -376,10 +377,10 @@ template <typename T> static int potential_t(dft_ot_functional *otf, cgrid *Pg, 
       if (base) p.x += base[i];
       T st = 0, dr[3] = { 0, 0, 0 };
       if (kc) {
-        st = (T) 1 - rt[i] * irs;
+        st = ((T) 1 - rt[i] * irs) * inv2h;
         for (int a = 0; a < 3; a++) {
           int ip, im; S.nb(x, y, z, i, a, ip, im);
-          dr[a] = (rho[ip] - rho[im]) * inv2h;
+          dr[a] = rho[ip] - rho[im];
         }
       }
       T va[3] = { 0, 0, 0 };
@@ -404,10 +405,10 @@ template <typename T> static int potential_t(dft_ot_functional *otf, cgrid *Pg, 
       }
       // src/ot.c:557-567 (the LJ term src/ot.c:530 is in the merged linear part)
       p.x += add;
-      if (loc) p.x += (c2 / (T) 2) * (b * b) + (c3 / (T) 3) * (b * b * b);
+      if (loc) p.x += (b * b) * (c2h + c3t * b);
       if (hdp) p.x += hp.vhd(rh);   // Barranco penalty src/ot.c:374-378, 815-819
       pot[i] = p;
-      if (loc) q[i] = (c2 * b + c3 * (b * b)) * rh;
+      if (loc) q[i] = (b * (c2 + c3 * b)) * rh;
       if (kc) {  // src/ot.c:608-612, 632-637 (rho_st itself is recomputed from rt where needed)
         s0[i] = dr[0] * st; s1[i] = dr[1] * st; s2[i] = dr[2] * st;
       }
@@ -472,7 +473,7 @@ template <typename T> static int potential_t(dft_ot_functional *otf, cgrid *Pg, 
   if (kc || bf) {
     const T c = (T) (otf->alpha_s / (2.0 * otf->mass)), hm = (T) (-0.5 * otf->mass), cbf = (T) otf->c_bfpot;
     const T pcap = (T) otf->max_bfpot, inv2h = (T) (1.0 / (2.0 * P->step));
-    const T eps = (T) otf->div_epsilon, irs = (T) (1.0 / otf->rho_0s);
+    const T eps = (T) otf->div_epsilon, irs = (T) (1.0 / otf->rho_0s), ch = c * inv2h;
     T *rt = r[R_RT], *J0 = r[R_J0], *J1 = r[R_J1], *J2 = r[R_J2], *h = r[R_H];
     T *v0 = r[R_V0], *v1 = r[R_V1], *v2 = r[R_V2], *A = r[R_A], *Cc = r[R_C], *B0 = r[R_BB0], *B1 = r[R_BB1], *B2 = r[R_BB2];
     T *wo0 = (T *) src.wout[0], *wo1 = (T *) src.wout[1], *wo2 = (T *) src.wout[2];
@@ -500,17 +501,17 @@ template <typename T> static int potential_t(dft_ot_functional *otf, cgrid *Pg, 
       T hval = 0, wv[3] = { 0, 0, 0 };   // stores last: every load is issued before them
       if (kc) {  // src/ot.c:641-645, 656-657, 673-675 summed over axes
         const T *Ja[3] = { J0, J1, J2 };
-        T hv = 0, t1 = 0, jd = 0;
+        T hv = 0, t1 = 0, jd = 0;   // times 2h
         for (int a = 0; a < 3; a++) {
           int ip, im; S.nb(x, y, z, i, a, ip, im);
           const T ja = Ja[a][i];
-          hv += (rho[ip] - rho[im]) * inv2h * ja;        // (d_a rho) J_a
-          t1 += (Ja[a][ip] - Ja[a][im]) * inv2h;         // dF_a * G_a = D_a J_a
-          jd += ja * ((rt[ip] - rt[im]) * inv2h);        // J_a (dF_a * rho) = J_a D_a (F*rho)
+          hv += (rho[ip] - rho[im]) * ja;                // (d_a rho) J_a
+          t1 += Ja[a][ip] - Ja[a][im];                   // dF_a * G_a = D_a J_a
+          jd += ja * (rt[ip] - rt[im]);                  // J_a (dF_a * rho) = J_a D_a (F*rho)
         }
         const T st = (T) 1 - rt[i] * irs;   // rho_st (src/ot.c:608-612)
-        p.x += c * st * t1 - c * jd;
-        hval = hv;
+        p.x += ch * (st * t1 - jd);
+        hval = hv * inv2h;
       }
       if (bf) {
         // real part src/ot.c:895-915 (V_j*(rho|v|^2) is in the linear part unless clamped)
@@ -528,15 +529,16 @@ template <typename T> static int potential_t(dft_ot_functional *otf, cgrid *Pg, 
         T rr = rho[i];
         const T gw = bfhd ? hp.g(rr) : (T) 1;
         if (rr < eps) rr = eps;
-        T im = 0;
+        T drw = 0, dw = 0;   // sum_a (D_a rho) w_a and sum_a D_a w_a, times 2h: one division a point
         for (int k = 0; k < 3; k++) {
           int ip, imm; S.nb(x, y, z, i, k, ip, imm);
           const T w = va[k][i] * a - Ba[k][i];
           wv[k] = w;
           const T wp = va[k][ip] * A[ip] - Ba[k][ip], wm = va[k][imm] * A[imm] - Ba[k][imm];
-          const T dr = bfhd ? hp.rg(rho[ip]) - hp.rg(rho[imm]) : rho[ip] - rho[imm];
-          im += (T) 0.5 * ((dr * inv2h) / rr) * w + (T) 0.5 * ((wp - wm) * inv2h) * gw;
+          drw += (bfhd ? hp.rg(rho[ip]) - hp.rg(rho[imm]) : rho[ip] - rho[imm]) * w;
+          dw += wp - wm;
         }
+        T im = (T) 0.5 * inv2h * (drw / rr + dw * gw);
         if (clampp) im = clampv<T>(im, pcap);
         p.y += im * cbf;
       }
@@ -657,7 +659,8 @@ template <typename T> static int energy_density_t(dft_ot_functional *otf, rgrid 
     DFT_TRY(F.inv_n(n, sp, dst));
   }
   {
-    const T c2 = (T) otf->c2, c3 = (T) otf->c3, irs = (T) (1.0 / otf->rho_0s), inv2h = (T) (1.0 / (2.0 * P->step));
+    const T c2h = (T) otf->c2 / (T) 2, c3t = (T) otf->c3 / (T) 3;
+    const T irs = (T) (1.0 / otf->rho_0s), inv2h = (T) (1.0 / (2.0 * P->step));
     const T cm = (T) (otf->c_bfpot * otf->mass);
     const double vf = 1.0 / (gwf->mass * 2.0 * P->step);
     T *u = r[R_U], *rb = r[R_RB], *rt = r[R_RT], *A = r[R_A], *rst = r[R_RST], *s0 = r[R_S0], *s1 = r[R_S1], *s2 = r[R_S2];
@@ -667,7 +670,7 @@ template <typename T> static int energy_density_t(dft_ot_functional *otf, rgrid 
       T acc = add ? ed[i] : (T) 0;
       if (plain) {  // src/ot-energy.c:70-93
         const T b = rb[i];
-        acc += (T) 0.5 * rh * u[i] + (c2 / (T) 2) * ((b * b) * rh) + (c3 / (T) 3) * ((b * b * b) * rh);
+        acc += rh * ((T) 0.5 * u[i] + (b * b) * (c2h + c3t * b));
       }
       if (hde) acc += hp.ehd(rh);   // src/ot-energy.c:96-99
       if (bosee) acc += bg.energy(rh);   // src/ot-energy.c:101-105
