@@ -410,6 +410,7 @@ __device__ __forceinline__ void line_body(const C *__restrict__ tw, const C *__r
   const int l = MAP == MAP_E ? threadIdx.x / TL : threadIdx.x % B;
   bool ok = true;
   C v[E];
+  pdl_begin();
   if constexpr (LDS == 0 && split_of<Ld>(0)) {
     typename Ld::Raw raw[E];
 #pragma unroll
@@ -685,6 +686,7 @@ __global__ void __launch_bounds__(256, MODE == 1 ? 1 : (MODE == 0 ? 3 : 2)) xcon
   }
   cp_async_commit();
   const size_t plane = (size_t) A.nx * A.ny;
+  pdl_begin();   // the kernel octants and the parameters above are constant
   if constexpr (MODE == 2) {
     C acc[E], v[E];
 #pragma unroll
@@ -816,6 +818,7 @@ __global__ void __launch_bounds__(256) xkinetic_kernel(const C *__restrict__ tw,
   }
   C *base = data + kz * (size_t) N * ny + y;
   C v[E];
+  pdl_begin();
 #pragma unroll
   for (int q = 0; q < E; q++) v[q] = base[(size_t) (t + TL * q) * ny];
   transform<N>(v, t, l, -1.f, tw, sm);

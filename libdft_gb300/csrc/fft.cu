@@ -352,9 +352,9 @@ template <int N> int fast_xconv(const XConvArgs<float> &A) {
   }
   ProfScope prof("fft_x_conv", xconv_bytes(A, F.kxh, F.kyh));
   const dim3 grid(A.ny / B, A.nkz, F.split ? A.nout : 1);
-  if (mode == 2) ff::xconv_kernel<N, 2><<<grid, 256, smem, rt().stream>>>(p.tw, F, multi);
-  else if (mode == 1) ff::xconv_kernel<N, 1><<<grid, 256, smem, rt().stream>>>(p.tw, F, multi);
-  else ff::xconv_kernel<N, 0><<<grid, 256, smem, rt().stream>>>(p.tw, F, multi);
+  if (mode == 2) launch_pdl(ff::xconv_kernel<N, 2>, grid, 256, smem, rt().stream, p.tw, F, multi);
+  else if (mode == 1) launch_pdl(ff::xconv_kernel<N, 1>, grid, 256, smem, rt().stream, p.tw, F, multi);
+  else launch_pdl(ff::xconv_kernel<N, 0>, grid, 256, smem, rt().stream, p.tw, F, multi);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }
@@ -366,7 +366,7 @@ template <int N> int fast_xkinetic(const KinArgs<float> &A) {
   DFT_TRY(get_plan<float>(N, &p));
   ProfScope prof("fft_x_kinetic", 2.0 * A.nx * A.ny * A.nz * sizeof(float2));
   auto k = A.cn ? ff::xkinetic_kernel<N, true> : ff::xkinetic_kernel<N, false>;
-  k<<<dim3(A.ny / B, A.nz), 256, 0, rt().stream>>>(
+  launch_pdl(k, dim3(A.ny / B, A.nz), 256, 0, rt().stream,
       p.tw, A.data, A.ny, A.nz, make_float2((float) A.cdt.x, (float) A.cdt.y), (float) A.inv_n, (float) A.dkx,
       (float) A.dky, (float) A.dkz, (float) A.kx0, (float) A.ky0, (float) A.kz0, (float) A.h);
   DFT_CHECK_LAUNCH();
@@ -422,7 +422,7 @@ template <typename T> int launch_xconv(XConvArgs<T> &A) {
   }
   ProfScope prof("fft_x_conv", bytes);
   if (A.nx == 1) {
-    xconv_point_kernel<T><<<(A.nkz * A.ny + 127) / 128, 128, 0, rt().stream>>>(A);
+    launch_pdl(xconv_point_kernel<T>, (A.nkz * A.ny + 127) / 128, 128, 0, rt().stream, A);
     DFT_CHECK_LAUNCH();
     return DFTGPU_OK;
   }
@@ -435,7 +435,7 @@ template <typename T> int launch_xconv(XConvArgs<T> &A) {
     DFT_CUDA(cudaFuncSetAttribute(xconv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) max_smem()));
     attr = true;
   }
-  xconv_kernel<T><<<dim3((A.ny + t.B - 1) / t.B, A.nkz, A.split ? A.nout : 1), t.threads, t.smem, rt().stream>>>(A);
+  launch_pdl(xconv_kernel<T>, dim3((A.ny + t.B - 1) / t.B, A.nkz, A.split ? A.nout : 1), t.threads, t.smem, rt().stream, A);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }

@@ -490,6 +490,7 @@ __global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 3 : 2)
   C *buf0 = reinterpret_cast<C *>(smem_raw), *buf1 = buf0 + args.B * g.LP;
   const FftPlan<T> &pl = args.plan;
   auto none = [](int, int, C) {};
+  pdl_begin();
 
   if constexpr (MODE == LINE_C2R) {
     // Z[k] = sum + i w^-k dif, sum, dif = X[k] +- X*[n-k], w = exp(-2 pi i / 2n),
@@ -624,6 +625,7 @@ __global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 3 : 2) xconv_ker
   const int tile = A.B * g.LP, ns = A.plan.nst;
   C *X = reinterpret_cast<C *>(smem_raw), *W = X + tile, *V = W + (ns >= 3 ? tile : 0), *ACC = V + tile;
   const size_t off = (size_t) kz * A.nx * A.ny + y0;
+  pdl_begin();
   const bool odd = (ns & 1) || ns == 0;   // the number of stage writes: the forward result ends in X
   auto none = [](int, int, C) {};
   int cur = -1;
@@ -676,6 +678,7 @@ __global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 3 : 2) xconv_ker
 // nx = 1: the x transforms are the identity
 template <typename T> __global__ void xconv_point_kernel(const __grid_constant__ XConvArgs<T> A) {
   typedef typename cplx_t<T>::type C;
+  pdl_begin();
   const size_t n = (size_t) A.nkz * A.ny;
   for (size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t) gridDim.x * blockDim.x) {
     const int kz = (int) (i / A.ny), y = (int) (i - (size_t) kz * A.ny);
@@ -751,6 +754,7 @@ __global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 3 : 2) xkinetic_
   C *X = reinterpret_cast<C *>(smem_raw), *W = X + tile, *fx = W + tile, *fyz = fx + n;
   C *base = A.data + (size_t) kz * A.nx * A.ny + y0;
   const C c = mk<T>((T) A.cdt.x, (T) A.cdt.y);
+  pdl_trigger();
   for (int e = threadIdx.x; e < n; e += blockDim.x) {
     const double k = kfreq(e, A.nx, A.dkx) - A.kx0, q = k * k;
     fx[e] = A.cn ? cn_m1(c, (T) k, (T) A.h) : cexpm1(mk<T>((T) (A.cdt.x * q), (T) (A.cdt.y * q)));
@@ -764,6 +768,7 @@ __global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 3 : 2) xkinetic_
   const int ns = A.plan.nst;
   const bool odd = (ns & 1) || ns == 0;
   auto none = [](int, int, C) {};
+  pdl_wait();
   tile_fft<false, T>(A.plan, g, 0, 0, odd ? X : W, odd ? W : X,
                      [&](int l, int e) { return base[(size_t) e * A.ny + l]; }, none);   // its barriers cover the tables
   const T inv_n = (T) A.inv_n;
@@ -850,13 +855,13 @@ void launch_line_kernel(int na, int nb, int nf, const float2 *tw, const float2 *
   const dim3 grid(nb / B, na, nf);
   if constexpr (LDS == 0 && ff::split_of<Ld>(0)) {
     auto k = ff::line_kernel_split<N, MODE, MAP, LDS, STS, TMA, NB, Ld, St>;
-    k<<<grid, 256, 0, rt().stream>>>(tw, tw2, sign, ld, st, resident_ctas(k), tm, fault);
+    launch_pdl(k, grid, 256, 0, rt().stream, tw, tw2, sign, ld, st, resident_ctas(k), tm, fault);
   } else if constexpr (STS == 0 && ff::bounded_store_of<St>(0)) {
     auto k = ff::line_kernel_stsplit<N, MODE, MAP, LDS, STS, TMA, NB, Ld, St>;
-    k<<<grid, 256, 0, rt().stream>>>(tw, tw2, sign, ld, st, resident_ctas(k), tm, fault);
+    launch_pdl(k, grid, 256, 0, rt().stream, tw, tw2, sign, ld, st, resident_ctas(k), tm, fault);
   } else {
     auto k = ff::line_kernel<N, MODE, MAP, LDS, STS, TMA, NB, Ld, St>;
-    k<<<grid, 256, 0, rt().stream>>>(tw, tw2, sign, ld, st, resident_ctas(k), tm, fault);
+    launch_pdl(k, grid, 256, 0, rt().stream, tw, tw2, sign, ld, st, resident_ctas(k), tm, fault);
   }
 }
 
@@ -964,7 +969,7 @@ int launch_generic_lines(const FftPlan<T> &plan, const typename cplx_t<T>::type 
     DFT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) max_smem()));
     Flag::done = true;
   }
-  kfn<<<dim3((nb + t.B - 1) / t.B, na, nf), t.threads, t.smem, stream>>>(args, ld, st);
+  launch_pdl(kfn, dim3((nb + t.B - 1) / t.B, na, nf), t.threads, t.smem, stream, args, ld, st);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }
@@ -1031,7 +1036,7 @@ template <typename T> int launch_generic_xkinetic(KinArgs<T> &A, cudaStream_t st
     DFT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) max_smem()));
     Flag::done = true;
   }
-  kfn<<<dim3((A.ny + t.B - 1) / t.B, A.nz), t.threads, t.smem, stream>>>(A);
+  launch_pdl(kfn, dim3((A.ny + t.B - 1) / t.B, A.nz), t.threads, t.smem, stream, A);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }

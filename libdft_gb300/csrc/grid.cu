@@ -510,6 +510,7 @@ int norm_dev(cgrid *c, double *slot) {
 // psi *= sqrt(target / norm) with norm read from the device slot
 // factor sqrt(target / norm) computed once in FP64, stored in the grid's precision
 template <typename T> __global__ void norm_factor_kernel(const double *slot, double target, T *factor) {
+  pdl_begin();
   *factor = (T) sqrt(target / slot[0]);
 }
 
@@ -519,7 +520,7 @@ template <typename T> int scale_by_norm_t(cgrid *c, const double *slot, double t
   T *factor = (T *) (reduce_slots() + 48);   // scratch slot, written here and read below on the same stream
   {
     ProfScope prof("reduce_fp64", 0.0);
-    norm_factor_kernel<T><<<1, 1, 0, rt().stream>>>(slot, target, factor);
+    launch_pdl(norm_factor_kernel<T>, 1, 1, 0, rt().stream, slot, target, factor);
     DFT_CHECK_LAUNCH();
   }
   return launch_each(gsize(c), [=] __device__(size_t i) {

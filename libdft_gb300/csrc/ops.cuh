@@ -8,6 +8,7 @@ namespace dftgpu {
 
 // grid-stride elementwise launch of a device lambda f(i), i < n
 template <class F> __global__ void each_kernel(size_t n, F f) {
+  pdl_begin();
   for (size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t) gridDim.x * blockDim.x) f(i);
 }
 
@@ -54,7 +55,7 @@ template <class F> int launch_each(size_t n, F f, double bytes = 0.0, const char
   int cap = rt().num_sms * 8;
   if (blocks > cap) blocks = cap;
   ProfScope prof(name, bytes);
-  each_kernel<<<blocks, 256, 0, rt().stream>>>(n, f);
+  launch_pdl(each_kernel<F>, blocks, 256, 0, rt().stream, n, f);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }
@@ -72,6 +73,7 @@ inline RowShape row_shape(int nx, int ny, int nz) {
   return RowShape{ dim3(ny, nx, (nz + bd - 1) / bd), bd };
 }
 template <class F> __global__ void rows_kernel(int ny, int nz, F f) {
+  pdl_begin();
   const int y = blockIdx.x, x = blockIdx.y, z = blockIdx.z * blockDim.x + threadIdx.x;
   if (z < nz) f(x, y, z, (x * ny + y) * nz + z);
 }
@@ -79,7 +81,7 @@ template <class F> __global__ void rows_kernel(int ny, int nz, F f) {
 template <class F> int launch_rows(int nx, int ny, int nz, F f, double bytes = 0.0, const char *name = "pointwise") {
   const RowShape r = row_shape(nx, ny, nz);
   ProfScope prof(name, bytes);
-  rows_kernel<<<r.grid, r.bd, 0, rt().stream>>>(ny, nz, f);
+  launch_pdl(rows_kernel<F>, r.grid, r.bd, 0, rt().stream, ny, nz, f);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }
@@ -87,6 +89,7 @@ template <class F> int launch_rows(int nx, int ny, int nz, F f, double bytes = 0
 // The same with a register budget for MINB resident 256-thread CTAs per SM:
 // for latency-bound passes with many independent loads per element.
 template <int MINB, class F> __global__ void __launch_bounds__(256, MINB) rows_kernel_b(int ny, int nz, F f) {
+  pdl_begin();
   const int y = blockIdx.x, x = blockIdx.y, z = blockIdx.z * blockDim.x + threadIdx.x;
   if (z < nz) f(x, y, z, (x * ny + y) * nz + z);
 }
@@ -94,7 +97,7 @@ template <int MINB, class F>
 int launch_rows_b(int nx, int ny, int nz, F f, double bytes = 0.0, const char *name = "pointwise") {
   const RowShape r = row_shape(nx, ny, nz);
   ProfScope prof(name, bytes);
-  rows_kernel_b<MINB><<<r.grid, r.bd, 0, rt().stream>>>(ny, nz, f);
+  launch_pdl(rows_kernel_b<MINB, F>, r.grid, r.bd, 0, rt().stream, ny, nz, f);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }
@@ -139,6 +142,7 @@ __device__ __forceinline__ double block_sum(double v) {
 }
 
 template <int NV, class F> __global__ void reduce_partial_kernel(size_t n, F f, double *partial) {
+  pdl_begin();
   double acc[NV];
 #pragma unroll
   for (int j = 0; j < NV; j++) acc[j] = 0.0;
@@ -156,6 +160,7 @@ template <int NV, class F> __global__ void reduce_partial_kernel(size_t n, F f, 
 }
 
 template <int NV> __global__ void reduce_final_kernel(const double *partial, double *slot, double scale) {
+  pdl_begin();
 #pragma unroll
   for (int j = 0; j < NV; j++) {
     double acc = 0.0;
@@ -170,9 +175,9 @@ template <int NV, class F> int reduce_dev(size_t n, F f, double *slot, double sc
   double *part; size_t np;
   DFT_TRY(reduce_partials(&part, &np));
   ProfScope prof("reduce_fp64", 0.0, 2);
-  reduce_partial_kernel<NV><<<RED_BLOCKS, RED_THREADS, 0, rt().stream>>>(n, f, part);
+  launch_pdl(reduce_partial_kernel<NV, F>, RED_BLOCKS, RED_THREADS, 0, rt().stream, n, f, part);
   DFT_CHECK_LAUNCH();
-  reduce_final_kernel<NV><<<1, RED_THREADS, 0, rt().stream>>>(part, slot, scale);
+  launch_pdl(reduce_final_kernel<NV>, 1, RED_THREADS, 0, rt().stream, part, slot, scale);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }

@@ -42,6 +42,7 @@ constexpr int march2_minb(int nt, bool kc, bool bf) { return nt >= 512 ? 1 : (kc
 // NT threads = nz; TY rows per CTA; KC / BF: the terms present
 template <int NT, int TY, bool KC, bool BF>
 __global__ void __launch_bounds__(NT, march2_minb(NT, KC, BF)) march2_kernel(const March2Args a) {
+  pdl_begin();
   static_assert(KC || BF, "one of the terms");
   // z-exchange plane, double-buffered: rho, F*rho, J_z, w_z of each row
   __shared__ float zx[2][4][TY][NT];
@@ -200,7 +201,7 @@ template <int NT, int TY, bool KC, bool BF> int launch_march2_t(March2Args &A) {
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, NT, 0) != cudaSuccess || per_sm < 1) per_sm = 1;
   A.lx = march_lx(A.nx, A.ny / TY, per_sm * rt().num_sms);
   dim3 grid(A.ny / TY, (A.nx + A.lx - 1) / A.lx);
-  k<<<grid, NT, 0, rt().stream>>>(A);
+  launch_pdl(k, grid, NT, 0, rt().stream, A);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }
