@@ -96,8 +96,9 @@ static int ot_vjp_t(dft_ot_functional *otf, wf *gwf, const typename cplx_t<T>::t
     xc_out(A, s[1]); xc_term(A, 0, F.k(OT_SA), KER_EVEN, (T) 1);
     if (kc) { xc_out(A, s[2]); xc_term(A, 0, F.k(OT_F), KER_EVEN, (T) 1); }
     DFT_TRY(launch_xconv<T>(A));
-    DFT_TRY(F.inv(s[1], r[A_WG]));
-    if (kc) DFT_TRY(F.inv(s[2], r[A_GAM]));
+    C *sp[2] = { s[1], s[2] };
+    T *dst[2] = { r[A_WG], r[A_GAM] };
+    DFT_TRY(F.inv_n(kc ? 2 : 1, sp, dst));
   }
   // pointwise 1: X = gamma (c2 rb + c3 rb^2) + Wg (c2 + 2 c3 rb) rho ; lambda_loc = Wg (c2 rb + c3 rb^2)
   //   KC: Y = gamma rho_st, divZ = sum_a D_a (gamma J_a), lJ_a = c (Gam g_a - gamma D_a (F*rho))
@@ -136,21 +137,18 @@ static int ot_vjp_t(dft_ot_functional *otf, wf *gwf, const typename cplx_t<T>::t
   }
   if (kc) {
     const T ck = (T) (otf->alpha_s / (2.0 * otf->mass));
-    DFT_TRY(F.fwd(r[A_Y], s[4]));
-    DFT_TRY(F.fwd(r[A_Z0], s[5]));
-    for (int a = 0; a < 3; a++) DFT_TRY(F.fwd(r[A_LJ0 + a], s[8 + a]));
-    XConvArgs<T> A; xc_init(A, P);                                          // F*Y ; lacc += c F*divZ
-    xc_in(A, (const C *) s[4]);
-    xc_in(A, (const C *) s[5]);
+    const T *in[5] = { r[A_Y], r[A_Z0], r[A_LJ0], r[A_LJ1], r[A_LJ2] };
+    C *sp[5] = { s[4], s[5], s[8], s[9], s[10] };
+    DFT_TRY(F.fwd_n(5, in, sp));
+    XConvArgs<T> A; xc_init(A, P);                                          // F*Y ; lacc += c F*divZ ; F * lJ_a
+    for (int i = 0; i < 5; i++) xc_in(A, (const C *) sp[i]);
     xc_out(A, s[4]); xc_term(A, 0, F.k(OT_F), KER_EVEN, (T) 1);
     xc_out(A, lacc, 1); xc_term(A, 1, F.k(OT_F), KER_EVEN, ck);
+    for (int i = 2; i < 5; i++) { xc_out(A, sp[i]); xc_term(A, i, F.k(OT_F), KER_EVEN, (T) 1); }
     DFT_TRY(launch_xconv<T>(A));
-    XConvArgs<T> D; xc_init(D, P);                                          // F * lJ_a
-    for (int a = 0; a < 3; a++) xc_in(D, (const C *) s[8 + a]);
-    for (int a = 0; a < 3; a++) { xc_out(D, s[8 + a]); xc_term(D, a, F.k(OT_F), KER_EVEN, (T) 1); }
-    DFT_TRY(launch_xconv<T>(D));
-    DFT_TRY(F.inv(s[4], r[A_Q0]));
-    for (int a = 0; a < 3; a++) DFT_TRY(F.inv(s[8 + a], r[A_FLJ0 + a]));
+    C *sb[4] = { s[4], s[8], s[9], s[10] };
+    T *dst[4] = { r[A_Q0], r[A_FLJ0], r[A_FLJ1], r[A_FLJ2] };
+    DFT_TRY(F.inv_n(4, sb, dst));
     // pointwise 2: Q_a = dF_a*Y = D_a (F*Y) ; lG_a = -c Q_a + F*lJ_a ; lg_a = c Gam J_a + lG_a rho_st ;
     //              lst = c gamma sum_a D_a J_a + sum lG_a g_a
     {
@@ -244,19 +242,17 @@ static int ot_vjp_t(dft_ot_functional *otf, wf *gwf, const typename cplx_t<T>::t
       }
       loc[i] -= acc;
     }));
-    DFT_TRY(F.fwd(r[A_LA], s[3]));
-    DFT_TRY(F.fwd(r[A_LC], s[4]));
-    for (int a = 0; a < 3; a++) DFT_TRY(F.fwd(r[A_LB0 + a], s[5 + a]));
     {
-      XConvArgs<T> A; xc_init(A, P); xc_in(A, (const C *) s[3]);
+      const T *in[5] = { r[A_LA], r[A_LC], r[A_LB0], r[A_LB1], r[A_LB2] };
+      C *sp[5] = { s[3], s[4], s[5], s[6], s[7] };
+      T *dst[4] = { r[A_LCIN], r[A_LBIN0], r[A_LBIN1], r[A_LBIN2] };
+      DFT_TRY(F.fwd_n(5, in, sp));
+      XConvArgs<T> A; xc_init(A, P);
+      for (int i = 0; i < 5; i++) xc_in(A, (const C *) sp[i]);
       xc_out(A, lacc, 1); xc_term(A, 0, F.k(OT_VJ), KER_EVEN, (T) 1);    // + V_j * lambda_A
+      for (int i = 1; i < 5; i++) { xc_out(A, sp[i]); xc_term(A, i, F.k(OT_VJ), KER_EVEN, (T) 1); }
       DFT_TRY(launch_xconv<T>(A));
-      XConvArgs<T> B; xc_init(B, P);
-      for (int a = 0; a < 4; a++) xc_in(B, (const C *) s[4 + a]);
-      for (int a = 0; a < 4; a++) { xc_out(B, s[4 + a]); xc_term(B, a, F.k(OT_VJ), KER_EVEN, (T) 1); }
-      DFT_TRY(launch_xconv<T>(B));
-      DFT_TRY(F.inv(s[4], r[A_LCIN]));
-      for (int a = 0; a < 3; a++) DFT_TRY(F.inv(s[5 + a], r[A_LBIN0 + a]));
+      DFT_TRY(F.inv_n(4, sp + 1, dst));
     }
     // B3: lambda_loc += lCin |v|^2 + sum lBin_a v_a ; mu_a += 2 lCin rho v_a + lBin_a rho ;
     //     velocity adjoint: g += -i kappa_a D_a psi + 2 lrho_v psi, K_a = kappa_a psi stored
@@ -397,13 +393,11 @@ static int strang_vjp_t(wf *g, cgrid *V, double dr, double di, const cgrid *psi,
   AdjLoad<T> ld{(const C *) gin->value, (const C *) V->value, ny, nz, hr, hi};
   SpecStoreZ<T> sz{spec, nx, ny};
   DFT_TRY((launch_lines<T, LINE_C2C, 1, 0>(nz, nx, ny, (T) -1, ld, sz)));
-  DFT_TRY(ypass<T>(spec, nx, ny, nz, (T) -1));
   KinArgs<T> K;
   kin_args<T>(K, nx, ny, nz, V->step, make_double2(di / (2.0 * g->mass), dr / (2.0 * g->mass)),   // conj(-i dt / 2m)
               g->grid->kx0, g->grid->ky0, g->grid->kz0, spec);
   K.cn = g->propagator == WF_2ND_ORDER_CN;   // real Q: the conjugate factor is the factor of conj(c)
-  DFT_TRY(launch_xkinetic<T>(K));
-  DFT_TRY(ypass<T>(spec, nx, ny, nz, (T) 1));
+  DFT_TRY(kinetic_yxy<T>(K, spec));
   SpecLoadZ<T> lz{spec, nx, ny};
   AdjStore<T> st{(C *) gout->value, (const C *) gin->value, (const C *) psi->value, (const C *) psio->value,
                  (const C *) V->value, (C *) gamV->value, ny, nz, hr, hi, (T) (0.5 * dr), (T) (0.5 * di), (T) scale, acc};

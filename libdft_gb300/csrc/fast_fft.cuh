@@ -798,7 +798,7 @@ __global__ void __launch_bounds__(256, MODE == 1 ? 1 : (MODE == 0 ? 3 : 2)) xcon
 // the Crank-Nicolson factor of the finite-difference kinetic operator, one per
 // axis (cn_m1; h the grid step)
 template <int N, bool CN>
-__global__ void __launch_bounds__(256) xkinetic_kernel(const C *__restrict__ tw, C *data, int ny, int nz, float2 cdt,
+__global__ void __launch_bounds__(256) xkinetic_kernel(const C *__restrict__ tw, C *data, int ny, int nz, int kz0i, float2 cdt,
                                                       float inv_n, float dkx, float dky, float dkz, float kx0,
                                                       float ky0, float kz0, float h) {
   constexpr int E = Shape<N>::E, TL = Shape<N>::TL, B = Shape<N>::B, LP = Shape<N>::LP;
@@ -811,7 +811,8 @@ __global__ void __launch_bounds__(256) xkinetic_kernel(const C *__restrict__ tw,
   }
   C fyz;                // exp(cdt ((ky - ky0)^2 + (kz - kz0)^2)) - 1 of this thread's line
   {
-    const float kzv = (float) (kz < (nz + 1) / 2 ? kz : kz - nz) * dkz - kz0;
+    const int kzi = kz0i + kz;
+    const float kzv = (float) (kzi < (nz + 1) / 2 ? kzi : kzi - nz) * dkz - kz0;
     const float kyv = (float) (y < (ny + 1) / 2 ? y : y - ny) * dky - ky0;
     const float q = kyv * kyv + kzv * kzv;
     fyz = CN ? cprod1p(cn_m1(cdt, kyv, h), cn_m1(cdt, kzv, h)) : cexpm1(make_float2(cdt.x * q, cdt.y * q));

@@ -364,10 +364,10 @@ template <int N> int fast_xkinetic(const KinArgs<float> &A) {
   if (A.ny % B) return -1;
   FftPlan<float> p;
   DFT_TRY(get_plan<float>(N, &p));
-  ProfScope prof("fft_x_kinetic", 2.0 * A.nx * A.ny * A.nz * sizeof(float2));
+  ProfScope prof("fft_x_kinetic", 2.0 * A.nx * A.ny * A.nkz * sizeof(float2));
   auto k = A.cn ? ff::xkinetic_kernel<N, true> : ff::xkinetic_kernel<N, false>;
-  launch_pdl(k, dim3(A.ny / B, A.nz), 256, 0, rt().stream,
-      p.tw, A.data, A.ny, A.nz, make_float2((float) A.cdt.x, (float) A.cdt.y), (float) A.inv_n, (float) A.dkx,
+  launch_pdl(k, dim3(A.ny / B, A.nkz), 256, 0, rt().stream,
+      p.tw, A.data, A.ny, A.nz, A.kz0i, make_float2((float) A.cdt.x, (float) A.cdt.y), (float) A.inv_n, (float) A.dkx,
       (float) A.dky, (float) A.dkz, (float) A.kx0, (float) A.ky0, (float) A.kz0, (float) A.h);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
@@ -458,8 +458,8 @@ template <typename T> int launch_xkinetic(KinArgs<T> &A) {
       if (rc >= 0) return rc;
     }
   }
-  DFT_TRY(get_plan<T>(A.nx, &A.plan, small_pass(A.nx, A.nz, A.ny)));
-  ProfScope prof("fft_x_kinetic", 2.0 * A.nx * A.ny * A.nz * sizeof(C));
+  DFT_TRY(get_plan<T>(A.nx, &A.plan, small_pass(A.nx, A.nkz, A.ny)));
+  ProfScope prof("fft_x_kinetic", 2.0 * A.nx * A.ny * A.nkz * sizeof(C));
   return launch_generic_xkinetic<T>(A, rt().stream);
 }
 

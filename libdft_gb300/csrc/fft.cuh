@@ -714,6 +714,7 @@ template <typename T> __global__ void xconv_point_kernel(const __grid_constant__
 template <typename T> struct KinArgs {
   FftPlan<T> plan;
   int B, logB, nx, ny, nz;
+  int kz0i, nkz;        // planes kz0i .. kz0i + nkz - 1 of the spectrum, data at the first
   double2 cdt;          // -i dt / (2 m): factor = exp(cdt |k - k0|^2)
   double inv_n;
   double dkx, dky, dkz; // 2 pi / (n step)
@@ -727,6 +728,7 @@ template <typename T>
 inline void kin_args(KinArgs<T> &K, int nx, int ny, int nz, double step, double2 cdt, double kx0, double ky0,
                      double kz0, typename cplx_t<T>::type *data) {
   K.nx = nx; K.ny = ny; K.nz = nz;
+  K.kz0i = 0; K.nkz = nz;
   K.data = data;
   K.cdt = cdt;
   K.inv_n = 1.0 / ((double) nx * ny * nz);
@@ -759,7 +761,7 @@ __global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 3 : 2) xkinetic_
     const double k = kfreq(e, A.nx, A.dkx) - A.kx0, q = k * k;
     fx[e] = A.cn ? cn_m1(c, (T) k, (T) A.h) : cexpm1(mk<T>((T) (A.cdt.x * q), (T) (A.cdt.y * q)));
   }
-  const double kzv = kfreq(kz, A.nz, A.dkz) - A.kz0;
+  const double kzv = kfreq(A.kz0i + kz, A.nz, A.dkz) - A.kz0;
   for (int l = threadIdx.x; l < B; l += blockDim.x) {
     const double k = kfreq(y0 + l, A.ny, A.dky) - A.ky0, q = k * k + kzv * kzv;
     fyz[l] = A.cn ? cprod1p(cn_m1(c, (T) k, (T) A.h), cn_m1(c, (T) kzv, (T) A.h))
@@ -1027,7 +1029,7 @@ template <typename T> int launch_xkinetic(KinArgs<T> &A);
 template <typename T> int launch_generic_xkinetic(KinArgs<T> &A, cudaStream_t stream) {
   typedef typename cplx_t<T>::type C;
   TileShape t;
-  DFT_TRY(choose_tile(A.nx, max_radix(A.plan), A.nz, A.ny, sizeof(C), 2, true, (size_t) A.nx * sizeof(C), &t));
+  DFT_TRY(choose_tile(A.nx, max_radix(A.plan), A.nkz, A.ny, sizeof(C), 2, true, (size_t) A.nx * sizeof(C), &t));
   A.B = t.B;
   A.logB = t.logB;
   auto kfn = xkinetic_kernel<T>;
@@ -1036,7 +1038,7 @@ template <typename T> int launch_generic_xkinetic(KinArgs<T> &A, cudaStream_t st
     DFT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) max_smem()));
     Flag::done = true;
   }
-  launch_pdl(kfn, dim3((A.ny + t.B - 1) / t.B, A.nz), t.threads, t.smem, stream, A);
+  launch_pdl(kfn, dim3((A.ny + t.B - 1) / t.B, A.nkz), t.threads, t.smem, stream, A);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }

@@ -361,15 +361,13 @@ template <typename T> int strang(wf *g, cgrid *dst, cgrid *src, cgrid *V, double
   PhaseLoad<T> ld{(const C *) src->value, (const C *) V->value, ny, nz, hr, hi};
   SpecStoreZ<T> sz{spec, nx, ny};
   DFT_TRY((launch_lines<T, LINE_C2C, 1, 0>(nz, nx, ny, (T) -1, ld, sz)));
-  DFT_TRY(ypass<T>(spec, nx, ny, nz, (T) -1));
   KinArgs<T> K;
   const double m = g->mass;
   const cgrid *mg = g->grid;   // moving-background momentum of the wave function
   kin_args<T>(K, nx, ny, nz, src->step, make_double2(di / (2.0 * m), -dr / (2.0 * m)),   // -i dt / 2m
               mg->kx0, mg->ky0, mg->kz0, spec);
   K.cn = cn;
-  DFT_TRY(launch_xkinetic<T>(K));
-  DFT_TRY(ypass<T>(spec, nx, ny, nz, (T) 1));
+  DFT_TRY(kinetic_yxy<T>(K, spec));
   SpecLoadZ<T> lz{spec, nx, ny};
   PhaseStore<T> st{(C *) dst->value, (const C *) V->value, ny, nz, hr, hi};
   return launch_lines<T, LINE_C2C, 0, 1>(nz, nx, ny, (T) 1, lz, st);

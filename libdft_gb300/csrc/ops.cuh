@@ -324,7 +324,7 @@ int launch_yz_c2r(const float2 *spec, const RealPairStore<float> &st, int nx, in
 // y passes over nkz planes of nf spectral buffers (ny = 1: the identity)
 template <typename T>
 int ypass_batch(typename cplx_t<T>::type *const *spec, int nf, int nx, int ny, int nkz, T sign) {
-  if (ny == 1) return DFTGPU_OK;
+  if (ny == 1 || nf == 0) return DFTGPU_OK;
   Batch<SpecLineY<T>, LINE_BATCH> io;
   memset(&io, 0, sizeof(io));
   for (int i = 0; i < nf; i++) io.f[i] = SpecLineY<T>{spec[i], nx, ny};
@@ -360,29 +360,12 @@ int irfft_yz(typename cplx_t<T>::type *spec, const St &st, int nx, int ny, int n
   return launch_lines<T, LINE_C2R, 0, 1>(nz / 2, nx, ny, (T) 1, ld, st, extra_bytes);
 }
 
-// Fields transformed by one launch: all (up to LINE_BATCH) in FP64, whose
-// passes are bound by the FP64 pipe; in FP32 as many as keep the batch's
-// spectra in L2 between their z and y passes (the fused plane passes, when
-// selected, take one).  Full potential, FP32, us: 128^3 (8.5 MB a spectrum) 318
-// one at a time on two branches, 275 five at a time, 286 all eight; 160 x 150 x
-// 144 844 / 838 / 861; 192^3 (28 MB) 925 one at a time, 939 three.  Up to 64^3
-// the step is launch-bound and all go together (64^3 191 / 123).
-template <typename T> inline int batch_fields(int nx, int ny, int nz) {
-  if (sizeof(T) == 8) return LINE_BATCH;
-  if (!fused_zy_off()) return 1;
-  const double spec = 8.0 * (nz / 2 + 1) * nx * ny;
-  const int k = (int) (kBatchBytes / spec);
-  return k < 1 ? 1 : k > LINE_BATCH ? LINE_BATCH : k;
-}
-
-// The z and y passes of nf real fields, batch_fields() at a time, the batches
-// on parallel branches.
+// ---------------------------------------------------------------- z passes and convolutions
+// The z passes of nf real fields, up to LINE_BATCH in one launch.
 template <typename T>
-int rfft_zy_n(const T *const *f, typename cplx_t<T>::type *const *spec, int nf, int nx, int ny, int nz) {
-  const int k = batch_fields<T>(nx, ny, nz);
-  return par_for((nf + k - 1) / k, [&](int j) -> int {
-    const int i0 = j * k, m = nf - i0 < k ? nf - i0 : k;
-    if (m == 1) return rfft_zy<T>(RealPairLoad<T>{f[i0], ny, nz}, spec[i0], nx, ny, nz);
+int zpass_fwd_n(const T *const *f, typename cplx_t<T>::type *const *spec, int nf, int nx, int ny, int nz) {
+  for (int i0 = 0; i0 < nf; i0 += LINE_BATCH) {
+    const int m = nf - i0 < LINE_BATCH ? nf - i0 : LINE_BATCH;
     Batch<RealPairLoad<T>, LINE_BATCH> ld;
     Batch<SpecStoreZ<T>, LINE_BATCH> st;
     memset(&ld, 0, sizeof(ld));
@@ -392,15 +375,13 @@ int rfft_zy_n(const T *const *f, typename cplx_t<T>::type *const *spec, int nf, 
       st.f[i] = SpecStoreZ<T>{spec[i0 + i], nx, ny};
     }
     DFT_TRY((launch_lines_batch<T, LINE_R2C, 1, 0, LINE_BATCH>(nz / 2, nx, ny, m, (T) -1, ld, st)));
-    return ypass_batch<T>(spec + i0, m, nx, ny, nz / 2 + 1, (T) -1);
-  });
+  }
+  return DFTGPU_OK;
 }
 template <typename T>
-int irfft_yz_n(typename cplx_t<T>::type *const *spec, T *const *f, int nf, int nx, int ny, int nz) {
-  const int k = batch_fields<T>(nx, ny, nz);
-  return par_for((nf + k - 1) / k, [&](int j) -> int {
-    const int i0 = j * k, m = nf - i0 < k ? nf - i0 : k;
-    if (m == 1) return irfft_yz<T>(spec[i0], RealPairStore<T>{f[i0], ny, nz, (T) 1}, nx, ny, nz);
+int zpass_inv_n(typename cplx_t<T>::type *const *spec, T *const *f, int nf, int nx, int ny, int nz) {
+  for (int i0 = 0; i0 < nf; i0 += LINE_BATCH) {
+    const int m = nf - i0 < LINE_BATCH ? nf - i0 : LINE_BATCH;
     Batch<SpecLoadZ<T>, LINE_BATCH> ld;
     Batch<RealPairStore<T>, LINE_BATCH> st;
     memset(&ld, 0, sizeof(ld));
@@ -409,8 +390,74 @@ int irfft_yz_n(typename cplx_t<T>::type *const *spec, T *const *f, int nf, int n
       ld.f[i] = SpecLoadZ<T>{spec[i0 + i], nx, ny};
       st.f[i] = RealPairStore<T>{f[i0 + i], ny, nz, (T) 1};
     }
-    DFT_TRY(ypass_batch<T>(spec + i0, m, nx, ny, nz / 2 + 1, (T) 1));
-    return launch_lines_batch<T, LINE_C2R, 0, 1, LINE_BATCH>(nz / 2, nx, ny, m, (T) 1, ld, st);
+    DFT_TRY((launch_lines_batch<T, LINE_C2R, 0, 1, LINE_BATCH>(nz / 2, nx, ny, m, (T) 1, ld, st)));
+  }
+  return DFTGPU_OK;
+}
+
+// Convolution of half spectra whose y passes are still to be done: forward y
+// passes of the inputs (those in the bit mask ydone have had theirs), x passes
+// of A, inverse y passes of the outputs.  Outputs may be inputs, not accumulate.
+// FP32 above kBatchBytes of spectra: the two halves of the kz planes on two
+// parallel branches, whose launches fill each other's last waves.  Full
+// potential, us, in one piece / halves / thirds: 128^3 258 / 252 / 261, 192^3
+// 906 / 896 / 927, 256^3 1753 / 1724 / 1749, 512 x 512 x 256 7642 / 7591 / 7659
+// (chunks small enough to stay in L2 between the passes: 1732 to 1789 and 8109
+// to 8214, their launches are too short).
+template <typename T> int convolve(const XConvArgs<T> &A, unsigned ydone) {
+  typedef typename cplx_t<T>::type C;
+  const size_t plane = (size_t) A.nx * A.ny, oct = (size_t) (A.nx / 2 + 1) * (A.ny / 2 + 1);
+  int extra = 0;   // outputs that are not inputs
+  for (int o = 0; o < A.nout; o++) {
+    bool in = false;
+    for (int i = 0; i < A.nin; i++) in |= A.out[o].dst == A.src[i];
+    extra += !in;
+  }
+  int step = A.nkz;
+  if (sizeof(T) == 4 && (double) (A.nin + extra) * plane * sizeof(C) * A.nkz > kBatchBytes) step = (A.nkz + 1) / 2;
+  return par_for((A.nkz + step - 1) / step, [&](int j) -> int {
+    const int k0 = j * step, nk = A.nkz - k0 < step ? A.nkz - k0 : step;
+    XConvArgs<T> c = A;
+    c.nkz = nk;
+    C *y[XC_MAX_OUT];
+    int n = 0;
+    for (int i = 0; i < A.nin; i++) {
+      c.src[i] = A.src[i] + k0 * plane;
+      if (!(ydone >> i & 1)) y[n++] = const_cast<C *>(c.src[i]);
+    }
+    for (int o = 0; o < A.nout; o++) {
+      c.out[o].dst = A.out[o].dst + k0 * plane;
+      for (int t = A.out[o].t0; t < A.out[o].t0 + A.out[o].nt; t++)
+        if (A.term[t].ker) c.term[t].ker = A.term[t].ker + k0 * oct;
+    }
+    DFT_TRY(ypass_batch<T>(y, n, A.nx, A.ny, nk, (T) -1));
+    DFT_TRY(launch_xconv<T>(c));
+    for (int o = 0; o < A.nout; o++) y[o] = c.out[o].dst;
+    return ypass_batch<T>(y, A.nout, A.nx, A.ny, nk, (T) 1);
+  });
+}
+
+// forward y, kinetic x and inverse y passes of a complex spectrum [nz][nx][ny],
+// in FP32 in chunks of planes that stay in L2 between the passes: one
+// propagation, us, whole / 80 / 40 / 20 MB chunks: 256^3 295 / 291 / 270 / 274,
+// 240^3 477 / 460 / 457 / 510, 512 x 512 x 256 1371 / 1381 / 1324 / 1300.
+constexpr double kKineticChunk = 40e6;
+template <typename T> int kinetic_yxy(const KinArgs<T> &K, typename cplx_t<T>::type *spec) {
+  const size_t plane = (size_t) K.nx * K.ny;
+  int step = K.nz;
+  const double bytes = (double) plane * 2 * sizeof(T) * K.nz;
+  if (sizeof(T) == 4 && bytes > kKineticChunk) {
+    const int n = (int) (bytes / kKineticChunk) + 1;
+    step = (K.nz + n - 1) / n;
+  }
+  return par_for((K.nz + step - 1) / step, [&](int j) -> int {
+    KinArgs<T> c = K;
+    c.kz0i = j * step;
+    c.nkz = K.nz - c.kz0i < step ? K.nz - c.kz0i : step;
+    c.data = spec + c.kz0i * plane;
+    DFT_TRY(ypass<T>(c.data, K.nx, K.ny, c.nkz, (T) -1));
+    DFT_TRY(launch_xkinetic<T>(c));
+    return ypass<T>(c.data, K.nx, K.ny, c.nkz, (T) 1);
   });
 }
 

@@ -326,17 +326,17 @@ template <typename T> static int potential_t(dft_ot_functional *otf, cgrid *Pg, 
   if (src.dens) {
     if (src.dens != otf->density->value)
       DFT_CUDA(cudaMemcpyAsync(rho, src.dens, nb, cudaMemcpyDeviceToDevice, rt().stream));
-    DFT_TRY(F.fwd(rho, s[0]));
+    DFT_TRY(F.zfwd(RealPairLoad<T>{rho, ny, nz}, s[0]));
   } else {   // rho = |psi|^2 (src/ot.c:320), formed and stored by the first z pass
     DensityPairLoad<T> ld{psi, rho, ny, nz};
-    DFT_TRY(rfft_zy<T>(ld, s[0], nx, ny, nz, 2.0 * nb));
+    DFT_TRY(F.zfwd(ld, s[0], 2.0 * nb));
   }
   // HD backflow: A = V_j * (rho G) (src/ot.c:843-849) convolves the cut-off density, s10
   const C *sA = s[0];
   if (bfhd) {
     T *rg = r[R_RG];
     DFT_TRY(launch_each((size_t) nx * ny * nz, [=] __device__(size_t i) { rg[i] = hp.rg(rho[i]); }, 2.0 * nb, "ot_hd_density"));
-    DFT_TRY(F.fwd(rg, s[10]));
+    DFT_TRY(F.zfwd(RealPairLoad<T>{rg, ny, nz}, s[10]));
     sA = s[10];
   }
 
@@ -350,12 +350,12 @@ template <typename T> static int potential_t(dft_ot_functional *otf, cgrid *Pg, 
     if (loc) { xc_out(A, s[2]); xc_term(A, 0, F.k(OT_SA), KER_EVEN, (T) 1); }
     if (kc) { xc_out(A, s[3]); xc_term(A, 0, F.k(OT_F), KER_EVEN, (T) 1); }
     if (bf) { xc_out(A, s[7]); xc_term(A, bfhd ? 1 : 0, F.k(OT_VJ), KER_EVEN, (T) 1); }
-    DFT_TRY(launch_xconv<T>(A));
+    DFT_TRY(F.conv(A));
     C *sp[3]; T *dst[3]; int n = 0;
     if (loc) { sp[n] = s[2]; dst[n++] = r[R_RB]; }
     if (kc) { sp[n] = s[3]; dst[n++] = r[R_RT]; }
     if (bf) { sp[n] = s[7]; dst[n++] = r[R_A]; }
-    DFT_TRY(F.inv_n(n, sp, dst));
+    DFT_TRY(F.zinv_n(n, sp, dst));
   }
 
   // pointwise 1
@@ -438,35 +438,27 @@ template <typename T> static int potential_t(dft_ot_functional *otf, cgrid *Pg, 
       in[n] = r[R_E]; sp[n++] = s[4];
       for (int a = 0; a < 3; a++) { in[n] = r[R_B0 + a]; sp[n++] = s[5 + a]; }
     }
-    DFT_TRY(F.fwd_n(n, in, sp));
+    DFT_TRY(F.zfwd_n(n, in, sp));
   }
 
   // x pass 2: J_a = F s_a^ (src/ot.c:652), B_a = V_j (rho v_a)^ and, when
-  // clamped, C = V_j (rho|v|^2)^, all in place.  The convolutions of one launch
-  // and the inverse transforms: all together where they are batched, else a
-  // KC and a BF chain on parallel branches.
-  {
-    C *sp[8]; T *dst[8]; const T *ker[8]; int n = 0, nkc = 0;
-    if (kc) for (int a = 0; a < 3; a++) { sp[n] = s[1 + a]; ker[n] = F.k(OT_F); dst[n++] = r[R_J0 + a]; }
-    nkc = n;
-    if (bf) {
-      for (int a = 0; a < 3; a++) { sp[n] = s[5 + a]; ker[n] = F.k(OT_VJ); dst[n++] = r[R_BB0 + a]; }
-      if (!cmerge) { sp[n] = s[4]; ker[n] = F.k(OT_VJ); dst[n++] = r[R_C]; }
-    }
-    auto chain = [&](int i0, int i1) -> int {
-      XConvArgs<T> A; xc_init(A, P);
-      for (int i = i0; i < i1; i++) xc_in(A, (const C *) sp[i]);
-      for (int i = i0; i < i1; i++) {
-        C *out = sp[i] == s[4] ? s[10] : sp[i];   // (rho|v|^2)^ is kept
-        xc_out(A, out); xc_term(A, i - i0, ker[i], KER_EVEN, (T) 1);
-        sp[i] = out;
-      }
-      DFT_TRY(launch_xconv<T>(A));
-      return F.inv_n(i1 - i0, sp + i0, dst + i0);
+  // clamped, C = V_j (rho|v|^2)^, in place
+  if (kc || bf) {
+    C *sp[8]; T *dst[8]; int n = 0;
+    XConvArgs<T> A; xc_init(A, P);
+    auto add = [&](C *in, C *out, const T *ker, T *field) {
+      xc_in(A, (const C *) in);
+      xc_out(A, out); xc_term(A, n, ker, KER_EVEN, (T) 1);
+      sp[n] = out;
+      dst[n++] = field;
     };
-    if (n > nkc && nkc > 0 && batch_fields<T>(nx, ny, nz) < n)
-      DFT_TRY(par_for(2, [&](int i) { return i == 0 ? chain(0, nkc) : chain(nkc, n); }));
-    else if (n > 0) DFT_TRY(chain(0, n));
+    if (kc) for (int a = 0; a < 3; a++) add(s[1 + a], s[1 + a], F.k(OT_F), r[R_J0 + a]);
+    if (bf) {
+      for (int a = 0; a < 3; a++) add(s[5 + a], s[5 + a], F.k(OT_VJ), r[R_BB0 + a]);
+      if (!cmerge) add(s[4], s[10], F.k(OT_VJ), r[R_C]);
+    }
+    DFT_TRY(F.conv(A));
+    DFT_TRY(F.zinv_n(n, sp, dst));
   }
 
   // pointwise 2
@@ -552,7 +544,7 @@ template <typename T> static int potential_t(dft_ot_functional *otf, cgrid *Pg, 
   //   V_LJ rho^ + w q^ (src/ot.c:530, 582-585) + c F h^ (KC, src/ot.c:656-664)
   //   + c_bf (-m/2) V_j (rho|v|^2)^ (BF, src/ot.c:895-915)
   const bool linear = lj || loc || kc || cmerge;
-  if (kc) DFT_TRY(F.fwd(r[R_H], s[10]));
+  if (kc) DFT_TRY(F.zfwd(RealPairLoad<T>{r[R_H], ny, nz}, s[10]));
   if (linear) {
     XConvArgs<T> A; xc_init(A, P);
     int nin = 0;
@@ -564,10 +556,10 @@ template <typename T> static int potential_t(dft_ot_functional *otf, cgrid *Pg, 
       xc_in(A, (const C *) s[4]);
       xc_term(A, nin++, F.k(OT_VJ), KER_EVEN, (T) (-0.5 * otf->mass * otf->c_bfpot));
     }
-    DFT_TRY(launch_xconv<T>(A));
+    DFT_TRY(F.conv(A, lj && (loc || kc || bf) ? 1u : 0u));   // rho^ (input 0) has been in x pass 1
     // P.re += linear part, P *= scale, in the store of the inverse transform
     PotAddPairStore<T> st{pot, ny, nz, scale};
-    return irfft_yz<T>(s[11], st, nx, ny, nz, 3.0 * nb);
+    return F.zinv(s[11], st, 3.0 * nb);
   }
 
   // pointwise 3 (no linear term): P *= scale
@@ -628,18 +620,18 @@ template <typename T> static int energy_density_t(dft_ot_functional *otf, rgrid 
   if (dens) {
     if (dens != otf->density) DFT_CUDA(cudaMemcpyAsync(rho, dens->value, nb, cudaMemcpyDeviceToDevice, rt().stream));
     if (!any) return add ? DFTGPU_OK : rfill(edg, 0.0);
-    DFT_TRY(F.fwd(rho, s[0]));
+    DFT_TRY(F.zfwd(RealPairLoad<T>{rho, ny, nz}, s[0]));
   } else if (!any) {
     DFT_TRY(density(gwf->grid, otf->density));
     return add ? DFTGPU_OK : rfill(edg, 0.0);
   } else {   // rho = |psi|^2 (src/ot-energy.c:44), formed and stored by the first z pass
     DensityPairLoad<T> ld{psi, rho, ny, nz};
-    DFT_TRY(rfft_zy<T>(ld, s[0], nx, ny, nz, 2.0 * nb));
+    DFT_TRY(F.zfwd(ld, s[0], 2.0 * nb));
   }
   T *rg = r[R_RG];   // the backflow's density: rho G(rho) (HD) or rho
   if (bfhd) {
     DFT_TRY(launch_each((size_t) nx * ny * nz, [=] __device__(size_t i) { rg[i] = hp.rg(rho[i]); }, 2.0 * nb, "ot_hd_density"));
-    DFT_TRY(F.fwd(rg, s[8]));
+    DFT_TRY(F.zfwd(RealPairLoad<T>{rg, ny, nz}, s[8]));
   }
   const T *rbf = bfhd ? rg : rho;
   if (plain || kc || bf) {
@@ -651,12 +643,12 @@ template <typename T> static int energy_density_t(dft_ot_functional *otf, rgrid 
     }
     if (kc) { xc_out(A, s[3]); xc_term(A, 0, F.k(OT_F), KER_EVEN, (T) 1); }
     if (bf) { xc_out(A, s[4]); xc_term(A, bfhd ? 1 : 0, F.k(OT_VJ), KER_EVEN, (T) 1); }
-    DFT_TRY(launch_xconv<T>(A));
+    DFT_TRY(F.conv(A));
     C *sp[4]; T *dst[4]; int n = 0;
     if (plain) { sp[n] = s[1]; dst[n++] = r[R_U]; sp[n] = s[2]; dst[n++] = r[R_RB]; }
     if (kc) { sp[n] = s[3]; dst[n++] = r[R_RT]; }
     if (bf) { sp[n] = s[4]; dst[n++] = r[R_A]; }
-    DFT_TRY(F.inv_n(n, sp, dst));
+    DFT_TRY(F.zinv_n(n, sp, dst));
   }
   {
     const T c2h = (T) otf->c2 / (T) 2, c3t = (T) otf->c3 / (T) 3;
@@ -708,11 +700,11 @@ template <typename T> static int energy_density_t(dft_ot_functional *otf, rgrid 
     XConvArgs<T> A; xc_init(A, P);
     if (kc) for (int a = 0; a < 3; a++) { in[n] = dst[n] = r[R_S0 + a]; sp[n++] = s[1 + a]; }
     if (bf) for (int a = 0; a < 4; a++) { in[n] = dst[n] = r[a == 0 ? R_E : R_B0 + a - 1]; sp[n++] = s[4 + a]; }
-    DFT_TRY(F.fwd_n(n, in, sp));
+    DFT_TRY(F.zfwd_n(n, in, sp));
     for (int i = 0; i < n; i++) xc_in(A, (const C *) sp[i]);
     for (int i = 0; i < n; i++) { xc_out(A, sp[i]); xc_term(A, i, F.k(kc && i < 3 ? OT_F : OT_VJ), KER_EVEN, (T) 1); }
-    DFT_TRY(launch_xconv<T>(A));
-    DFT_TRY(F.inv_n(n, sp, dst));
+    DFT_TRY(F.conv(A));
+    DFT_TRY(F.zinv_n(n, sp, dst));
   }
   if (kc || bf) {
     const T f = (T) (-otf->alpha_s / (4.0 * otf->mass)), cm = (T) (otf->c_bfpot * otf->mass);
