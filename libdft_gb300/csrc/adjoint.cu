@@ -479,8 +479,7 @@ static int fwd_step(dft_ot_functional *otf, AdjWork *W, const cgrid *src, cgrid 
   DFT_TRY(record_step(otf, W, vext, mu0, dr, di));
   if (renorm) {
     double *slot = reduce_slots();
-    DFT_TRY(norm_dev(W->psio, slot + 4));
-    DFT_TRY(scale_by_norm(W->psio, slot + 4, norm));
+    DFT_TRY(normalize(W->psio, slot + 4, norm));
   }
   return ccopy(dst, W->psio);
 }

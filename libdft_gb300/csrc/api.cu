@@ -429,8 +429,7 @@ REAL grid_wf_norm(wf *g) {
 REAL grid_wf_normalize(wf *g) {
   NEED(g, "grid_wf_normalize", NAN);
   double *slot = reduce_slots();
-  if (norm_dev(g->grid, slot + 2) != DFTGPU_OK) return NAN;
-  if (scale_by_norm(g->grid, slot + 2, g->norm) != DFTGPU_OK) return NAN;
+  if (normalize(g->grid, slot + 2, g->norm) != DFTGPU_OK) return NAN;
   double v = NAN;
   if (cudaMemcpyAsync(&v, slot + 2, sizeof(double), cudaMemcpyDeviceToHost, rt().stream) != cudaSuccess ||
       cudaStreamSynchronize(rt().stream) != cudaSuccess) { set_error(DFTGPU_ERR_CUDA, "grid_wf_normalize"); return NAN; }
@@ -868,8 +867,7 @@ static int step_with_renorm(dft_ot_functional *otf, wf *gwf, wf *gwfp, cgrid *P,
   DFT_TRY(pc_step_impl(otf, gwf, gwfp, P, vext, mu0, dr, di));
   if (renorm) {
     double *slot = reduce_slots();
-    DFT_TRY(norm_dev(gwf->grid, slot + 3));
-    DFT_TRY(scale_by_norm(gwf->grid, slot + 3, gwf->norm));
+    DFT_TRY(normalize(gwf->grid, slot + 3, gwf->norm));
   }
   return DFTGPU_OK;
 }

@@ -483,7 +483,7 @@ int kinetic_energy(wf *g, double *out) {
 // in the grid's precision (FP32: within 8 ulps of the run's sum), runs are
 // accumulated in FP64 -- one FP64 add per 8 values instead of per value.  The
 // last run is short when 8 does not divide the count (odd x and y sizes).
-template <typename T> int norm_dev_t(cgrid *c, double *slot) {
+template <typename T, class After> int norm_dev_t(cgrid *c, double *slot, After after) {
   typedef typename cplx_t<T>::type C;
   const C *p = (const C *) c->value;
   const double dv = c->step * c->step * c->step;
@@ -498,29 +498,23 @@ template <typename T> int norm_dev_t(cgrid *c, double *slot) {
       for (size_t k = 0; 8 * r + k < n; k++) { const C z = q[k]; s += z.x * z.x + z.y * z.y; }
     }
     v[0] = (double) s;
-  }, slot, dv);
+  }, slot, dv, after);
 }
 
 int norm_dev(cgrid *c, double *slot) {
-  return c->prec == DFTGPU_FP32 ? norm_dev_t<float>(c, slot) : norm_dev_t<double>(c, slot);
+  return c->prec == DFTGPU_FP32 ? norm_dev_t<float>(c, slot, NoAfter()) : norm_dev_t<double>(c, slot, NoAfter());
 }
 
-// psi *= sqrt(target / norm) with norm read from the device slot
-// factor sqrt(target / norm) computed once in FP64, stored in the grid's precision
-template <typename T> __global__ void norm_factor_kernel(const double *slot, double target, T *factor) {
-  pdl_begin();
-  *factor = (T) sqrt(target / slot[0]);
-}
-
-template <typename T> int scale_by_norm_t(cgrid *c, const double *slot, double target) {
+// norm into the device slot, then psi *= sqrt(target / norm): the factor is
+// formed once in FP64 by the reduction's last kernel and stored in the grid's
+// precision
+template <typename T> int normalize_t(cgrid *c, double *slot, double target) {
   typedef typename cplx_t<T>::type C;
   C *p = (C *) c->value;
-  T *factor = (T *) (reduce_slots() + 48);   // scratch slot, written here and read below on the same stream
-  {
-    ProfScope prof("reduce_fp64", 0.0);
-    launch_pdl(norm_factor_kernel<T>, 1, 1, 0, rt().stream, slot, target, factor);
-    DFT_CHECK_LAUNCH();
-  }
+  double *slots = reduce_slots();
+  if (!slots) { set_error(DFTGPU_ERR_NOMEM, "reduction slots"); return DFTGPU_ERR_NOMEM; }
+  T *factor = (T *) (slots + 48);   // scratch slot, written by the reduction and read below on the same stream
+  DFT_TRY(norm_dev_t<T>(c, slot, [=] __device__(const double *norm) { *factor = (T) sqrt(target / norm[0]); }));
   return launch_each(gsize(c), [=] __device__(size_t i) {
     const T f = *factor;
     C z = p[i];
@@ -529,8 +523,8 @@ template <typename T> int scale_by_norm_t(cgrid *c, const double *slot, double t
   }, 4.0 * gsize(c) * sizeof(T), "normalize");
 }
 
-int scale_by_norm(cgrid *c, const double *slot, double target) {
-  return c->prec == DFTGPU_FP32 ? scale_by_norm_t<float>(c, slot, target) : scale_by_norm_t<double>(c, slot, target);
+int normalize(cgrid *c, double *slot, double target) {
+  return c->prec == DFTGPU_FP32 ? normalize_t<float>(c, slot, target) : normalize_t<double>(c, slot, target);
 }
 
 template <typename T> int velocity_t(wf *g, rgrid *vx, rgrid *vy, rgrid *vz, double eps) {

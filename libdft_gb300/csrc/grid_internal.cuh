@@ -55,7 +55,7 @@ template <typename T> struct SpecLineXT {
 int propagate(wf *g, cgrid *dst, cgrid *src, cgrid *V, double dr, double di);
 int kinetic_energy(wf *g, double *out);
 int norm_dev(cgrid *c, double *slot);
-int scale_by_norm(cgrid *c, const double *slot, double target);
+int normalize(cgrid *c, double *slot, double target);   // norm into slot, then psi *= sqrt(target / norm)
 int velocity(wf *g, rgrid *vx, rgrid *vy, rgrid *vz, double eps);
 int copy_values_out(int prec, const void *dev, double *host, size_t n);
 int copy_values_in(int prec, void *dev, const double *host, size_t n);

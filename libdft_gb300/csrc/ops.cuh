@@ -65,23 +65,27 @@ template <class F> int launch_each(size_t n, F f, double bytes = 0.0, const char
 // with i the linear index, no index division.  Few rows (1-D grids: one) are
 // cut into segments of 32 values, one warp each, so that they use many SMs: a
 // 4096-point row's second OT pass took 150 us on one SM.
-struct RowShape { dim3 grid; int bd; };
+// Short rows share a CTA (up to 256 threads) while that leaves four CTAs per SM.
+struct RowShape { dim3 grid, block; };
 inline RowShape row_shape(int nx, int ny, int nz) {
   int nseg = (nz + 255) / 256;
   if ((size_t) nx * ny * nseg < (size_t) 2 * rt().num_sms) nseg = (nz + 31) / 32;
   const int bd = ((nz + nseg - 1) / nseg + 31) / 32 * 32;
-  return RowShape{ dim3(ny, nx, (nz + bd - 1) / bd), bd };
+  nseg = (nz + bd - 1) / bd;
+  int ry = 1;
+  while (2 * ry * bd <= 256 && (size_t) nx * nseg * ((ny + 2 * ry - 1) / (2 * ry)) >= (size_t) 4 * rt().num_sms) ry *= 2;
+  return RowShape{ dim3((ny + ry - 1) / ry, nx, nseg), dim3(bd, ry) };
 }
 template <class F> __global__ void rows_kernel(int ny, int nz, F f) {
   pdl_begin();
-  const int y = blockIdx.x, x = blockIdx.y, z = blockIdx.z * blockDim.x + threadIdx.x;
-  if (z < nz) f(x, y, z, (x * ny + y) * nz + z);
+  const int y = blockIdx.x * blockDim.y + threadIdx.y, x = blockIdx.y, z = blockIdx.z * blockDim.x + threadIdx.x;
+  if (y < ny && z < nz) f(x, y, z, (x * ny + y) * nz + z);
 }
 
 template <class F> int launch_rows(int nx, int ny, int nz, F f, double bytes = 0.0, const char *name = "pointwise") {
   const RowShape r = row_shape(nx, ny, nz);
   ProfScope prof(name, bytes);
-  launch_pdl(rows_kernel<F>, r.grid, r.bd, 0, rt().stream, ny, nz, f);
+  launch_pdl(rows_kernel<F>, r.grid, r.block, 0, rt().stream, ny, nz, f);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }
@@ -90,14 +94,14 @@ template <class F> int launch_rows(int nx, int ny, int nz, F f, double bytes = 0
 // for latency-bound passes with many independent loads per element.
 template <int MINB, class F> __global__ void __launch_bounds__(256, MINB) rows_kernel_b(int ny, int nz, F f) {
   pdl_begin();
-  const int y = blockIdx.x, x = blockIdx.y, z = blockIdx.z * blockDim.x + threadIdx.x;
-  if (z < nz) f(x, y, z, (x * ny + y) * nz + z);
+  const int y = blockIdx.x * blockDim.y + threadIdx.y, x = blockIdx.y, z = blockIdx.z * blockDim.x + threadIdx.x;
+  if (y < ny && z < nz) f(x, y, z, (x * ny + y) * nz + z);
 }
 template <int MINB, class F>
 int launch_rows_b(int nx, int ny, int nz, F f, double bytes = 0.0, const char *name = "pointwise") {
   const RowShape r = row_shape(nx, ny, nz);
   ProfScope prof(name, bytes);
-  launch_pdl(rows_kernel_b<MINB, F>, r.grid, r.bd, 0, rt().stream, ny, nz, f);
+  launch_pdl(rows_kernel_b<MINB, F>, r.grid, r.block, 0, rt().stream, ny, nz, f);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }
@@ -159,25 +163,32 @@ template <int NV, class F> __global__ void reduce_partial_kernel(size_t n, F f, 
   }
 }
 
-template <int NV> __global__ void reduce_final_kernel(const double *partial, double *slot, double scale) {
+// after(results) runs on one thread once the results are formed
+struct NoAfter { __device__ void operator()(const double *) const {} };
+template <int NV, class After>
+__global__ void reduce_final_kernel(const double *partial, double *slot, double scale, After after) {
   pdl_begin();
+  double res[NV];
 #pragma unroll
   for (int j = 0; j < NV; j++) {
     double acc = 0.0;
     for (int i = threadIdx.x; i < RED_BLOCKS; i += blockDim.x) acc += partial[j * RED_BLOCKS + i];
     double s = block_sum(acc);
-    if (threadIdx.x == 0) slot[j] = s * scale;
+    res[j] = s * scale;
+    if (threadIdx.x == 0) slot[j] = res[j];
   }
+  if (threadIdx.x == 0) after(res);
 }
 
 // f(i, double v[NV]); results (times scale) to slot[0..NV) on the device.
-template <int NV, class F> int reduce_dev(size_t n, F f, double *slot, double scale) {
+template <int NV, class F, class After = NoAfter>
+int reduce_dev(size_t n, F f, double *slot, double scale, After after = NoAfter()) {
   double *part; size_t np;
   DFT_TRY(reduce_partials(&part, &np));
   ProfScope prof("reduce_fp64", 0.0, 2);
   launch_pdl(reduce_partial_kernel<NV, F>, RED_BLOCKS, RED_THREADS, 0, rt().stream, n, f, part);
   DFT_CHECK_LAUNCH();
-  launch_pdl(reduce_final_kernel<NV>, 1, RED_THREADS, 0, rt().stream, part, slot, scale);
+  launch_pdl(reduce_final_kernel<NV, After>, 1, RED_THREADS, 0, rt().stream, part, slot, scale, after);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }
