@@ -282,8 +282,14 @@ done:
 // src selects the terms (LJ, local correlation, KC, BF) and where rho and v
 // come from: psi (dft_ot_potential) or given grids (dft_ot_potential2 and the
 // per-term entry points, src/ot.c:431-507, 524-586, 840-991).
+// The FP64 pointwise passes are bound by the FP64 pipe and take the forms with
+// the fewest operations; the FP32 ones are bound by memory and keep theirs
+// (their rounding decides how the FP32 norm drifts over long real-time runs).
+template <typename T> constexpr bool few_ops_v = sizeof(T) == 8;
+
 template <typename T> static int potential_t(dft_ot_functional *otf, cgrid *Pg, wf *gwf, int overwrite, const T *base,
                                              double add_d, double scale_d, const PotSrc &src) {
+  constexpr bool few_ops = few_ops_v<T>;
   const T add = (T) add_d, scale = (T) scale_d;
   typedef typename cplx_t<T>::type C;
   OtPriv *P = (OtPriv *) otf->priv;
@@ -377,10 +383,12 @@ template <typename T> static int potential_t(dft_ot_functional *otf, cgrid *Pg, 
       if (base) p.x += base[i];
       T st = 0, dr[3] = { 0, 0, 0 };
       if (kc) {
-        st = ((T) 1 - rt[i] * irs) * inv2h;
+        st = (T) 1 - rt[i] * irs;
+        if (few_ops) st *= inv2h;
         for (int a = 0; a < 3; a++) {
           int ip, im; S.nb(x, y, z, i, a, ip, im);
           dr[a] = rho[ip] - rho[im];
+          if (!few_ops) dr[a] *= inv2h;
         }
       }
       T va[3] = { 0, 0, 0 };
@@ -405,10 +413,10 @@ template <typename T> static int potential_t(dft_ot_functional *otf, cgrid *Pg, 
       }
       // src/ot.c:557-567 (the LJ term src/ot.c:530 is in the merged linear part)
       p.x += add;
-      if (loc) p.x += (b * b) * (c2h + c3t * b);
+      if (loc) p.x += few_ops ? (b * b) * (c2h + c3t * b) : c2h * (b * b) + c3t * (b * b * b);
       if (hdp) p.x += hp.vhd(rh);   // Barranco penalty src/ot.c:374-378, 815-819
       pot[i] = p;
-      if (loc) q[i] = (b * (c2 + c3 * b)) * rh;
+      if (loc) q[i] = (few_ops ? b * (c2 + c3 * b) : c2 * b + c3 * (b * b)) * rh;
       if (kc) {  // src/ot.c:608-612, 632-637 (rho_st itself is recomputed from rt where needed)
         s0[i] = dr[0] * st; s1[i] = dr[1] * st; s2[i] = dr[2] * st;
       }
@@ -493,17 +501,18 @@ template <typename T> static int potential_t(dft_ot_functional *otf, cgrid *Pg, 
       T hval = 0, wv[3] = { 0, 0, 0 };   // stores last: every load is issued before them
       if (kc) {  // src/ot.c:641-645, 656-657, 673-675 summed over axes
         const T *Ja[3] = { J0, J1, J2 };
-        T hv = 0, t1 = 0, jd = 0;   // times 2h
+        T hv = 0, t1 = 0, jd = 0;
+        const T k = few_ops ? (T) 1 : inv2h;             // few_ops: the sums times 2h
         for (int a = 0; a < 3; a++) {
           int ip, im; S.nb(x, y, z, i, a, ip, im);
           const T ja = Ja[a][i];
-          hv += (rho[ip] - rho[im]) * ja;                // (d_a rho) J_a
-          t1 += Ja[a][ip] - Ja[a][im];                   // dF_a * G_a = D_a J_a
-          jd += ja * (rt[ip] - rt[im]);                  // J_a (dF_a * rho) = J_a D_a (F*rho)
+          hv += (rho[ip] - rho[im]) * k * ja;            // (d_a rho) J_a
+          t1 += (Ja[a][ip] - Ja[a][im]) * k;             // dF_a * G_a = D_a J_a
+          jd += ja * ((rt[ip] - rt[im]) * k);            // J_a (dF_a * rho) = J_a D_a (F*rho)
         }
         const T st = (T) 1 - rt[i] * irs;   // rho_st (src/ot.c:608-612)
-        p.x += ch * (st * t1 - jd);
-        hval = hv * inv2h;
+        p.x += few_ops ? ch * (st * t1 - jd) : c * st * t1 - c * jd;
+        hval = few_ops ? hv * inv2h : hv;
       }
       if (bf) {
         // real part src/ot.c:895-915 (V_j*(rho|v|^2) is in the linear part unless clamped)
@@ -521,16 +530,21 @@ template <typename T> static int potential_t(dft_ot_functional *otf, cgrid *Pg, 
         T rr = rho[i];
         const T gw = bfhd ? hp.g(rr) : (T) 1;
         if (rr < eps) rr = eps;
-        T drw = 0, dw = 0;   // sum_a (D_a rho) w_a and sum_a D_a w_a, times 2h: one division a point
+        T im = 0, drw = 0, dw = 0;   // few_ops: sum_a (D_a rho) w_a and sum_a D_a w_a, times 2h: one division a point
         for (int k = 0; k < 3; k++) {
           int ip, imm; S.nb(x, y, z, i, k, ip, imm);
           const T w = va[k][i] * a - Ba[k][i];
           wv[k] = w;
           const T wp = va[k][ip] * A[ip] - Ba[k][ip], wm = va[k][imm] * A[imm] - Ba[k][imm];
-          drw += (bfhd ? hp.rg(rho[ip]) - hp.rg(rho[imm]) : rho[ip] - rho[imm]) * w;
-          dw += wp - wm;
+          const T dr = bfhd ? hp.rg(rho[ip]) - hp.rg(rho[imm]) : rho[ip] - rho[imm];
+          if (few_ops) {
+            drw += dr * w;
+            dw += wp - wm;
+          } else {
+            im += (T) 0.5 * ((dr * inv2h) / rr) * w + (T) 0.5 * ((wp - wm) * inv2h) * gw;
+          }
         }
-        T im = (T) 0.5 * inv2h * (drw / rr + dw * gw);
+        if (few_ops) im = (T) 0.5 * inv2h * (drw / rr + dw * gw);
         if (clampp) im = clampv<T>(im, pcap);
         p.y += im * cbf;
       }
@@ -594,6 +608,7 @@ int ot_potential_src(dft_ot_functional *otf, cgrid *P, wf *gwf, int overwrite, r
 // points add to the plain part, src/ot-energy.c:108-109).
 template <typename T> static int energy_density_t(dft_ot_functional *otf, rgrid *edg, wf *gwf, int terms,
                                                   const rgrid *dens, bool add) {
+  constexpr bool few_ops = few_ops_v<T>;
   typedef typename cplx_t<T>::type C;
   OtPriv *P = (OtPriv *) otf->priv;
   Fields<T> F{P, P->nx, P->ny, P->nz};
@@ -662,7 +677,8 @@ template <typename T> static int energy_density_t(dft_ot_functional *otf, rgrid 
       T acc = add ? ed[i] : (T) 0;
       if (plain) {  // src/ot-energy.c:70-93
         const T b = rb[i];
-        acc += rh * ((T) 0.5 * u[i] + (b * b) * (c2h + c3t * b));
+        acc += few_ops ? rh * ((T) 0.5 * u[i] + (b * b) * (c2h + c3t * b))
+                       : (T) 0.5 * rh * u[i] + c2h * ((b * b) * rh) + c3t * ((b * b * b) * rh);
       }
       if (hde) acc += hp.ehd(rh);   // src/ot-energy.c:96-99
       if (bosee) acc += bg.energy(rh);   // src/ot-energy.c:101-105
