@@ -62,8 +62,7 @@ template <typename T> int get_plan(int n, FftPlan<T> *plan, bool small = false);
 // radix 16 take 21.  Measured on full potentials, radices up to 5 against up
 // to 16 (us): 32^3 291 / 365, 64^3 517 / 541, 96 x 90 x 80 1452 / 1493, 128^3
 // (2^20 values a pass) 3259 / 3230, 160 x 150 x 144 7971 / 7295.
-// A few long lines (1-D grids) are bound by one SM's FP64 pipe instead.
-inline bool small_pass(int n, int na, int nb) { return (size_t) n * na * nb <= (size_t) 1 << 19 && na * nb >= 16; }
+inline bool small_pass(int n, int na, int nb) { return (size_t) n * na * nb <= (size_t) 1 << 19; }
 
 // ------------------------------------------------------------ butterflies
 template <typename C, typename T>
@@ -976,6 +975,145 @@ int launch_generic_lines(const FftPlan<T> &plan, const typename cplx_t<T>::type 
   return DFTGPU_OK;
 }
 
+// ------------------------------------------------------------ split lines
+// A long FP64 line is bound by one SM's FP64 pipe (n = 2048: 2048 x 30
+// operations at 2 per clock, 15 us, where the whole chip takes 0.1), and a 1-D
+// grid has one line a field.  So a single line of n = n1 n2 >= kSplitLine
+// values runs as two passes of short lines over many CTAs, through scratch of
+// its own length that follows the spectrum:
+//   pass 1: for every j2 the n1-point DFT over j1 of x[j1 n2 + j2], times
+//           exp(-2 pi i j2 k1 / n), to A[k1 n2 + j2]
+//   pass 2: for every k1 the n2-point DFT over j2, to X[k1 + n1 k2];
+// C2R forms its Z[k] in the loads of pass 1, R2C its X[k] in a third launch.
+// Inverse transforms run on (im, re).  A full real-time step of a 1-D grid, us,
+// one CTA a line / split: 4096 points 779 / 369, 2048 521 / 307, 1024 (real
+// transforms of 512) 316 / 270, propagation alone of 512 points 51 / 34; 256
+// points stay in one launch (29).
+constexpr int kSplitLine = 512;
+
+template <class F> struct SplitLoad {       // x[j1 n2 + j2] of line functor F
+  F ld; int n2, inverse;
+  __device__ auto operator()(int, int j2, int j1) const { return swap_if(ld(0, 0, j1 * n2 + j2), inverse); }
+};
+template <typename T, class F> struct SplitPre {   // Z[k] of the C2R transform of length n, as (im, re)
+  typedef typename cplx_t<T>::type C;
+  F ld; const C *tw2; int n, n2;
+  __device__ C operator()(int, int j2, int j1) const {
+    const int k = j1 * n2 + j2;
+    C xk = ld(0, 0, k), xm = ld(0, 0, n - k);
+    if (k == 0) { xk.y = (T) 0; xm.y = (T) 0; }
+    const C w = __ldg(&tw2[k]);
+    const T sx = xk.x + xm.x, sy = xk.y - xm.y, dx = xk.x - xm.x, dy = xk.y + xm.y;
+    return mk<T>(fma_t(dx, w.x, fma_t(dy, w.y, sy)), fma_t(dx, w.y, fma_t(-dy, w.x, sx)));
+  }
+};
+template <typename T> struct SplitMid {     // A[k1 n2 + j2]: pass 1 stores (line j2, element k1), pass 2 loads (line k1, element j2)
+  typedef typename cplx_t<T>::type C;
+  C *A; const C *tw; int n2;
+  __device__ void operator()(int, int j2, int k1, C v) const { A[k1 * n2 + j2] = cmul(v, __ldg(&tw[j2 * k1])); }
+  __device__ C operator()(int, int k1, int j2) const { return A[k1 * n2 + j2]; }
+};
+template <class F> struct SplitStore {      // X[k1 + n1 k2] of line functor F
+  F st; int n1, inverse;
+  template <typename C> __device__ void operator()(int, int k1, int k2, C v) const {
+    st(0, 0, k1 + n1 * k2, swap_if(v, inverse));
+  }
+};
+template <typename T> struct SplitPlain {   // R2C: Z into a plain array
+  typename cplx_t<T>::type *B;
+  __device__ void operator()(int, int, int k, typename cplx_t<T>::type v) const { B[k] = v; }
+};
+template <typename T, int NB, class St>
+__global__ void split_post_kernel(int n, const typename cplx_t<T>::type *__restrict__ tw2,
+                                  const __grid_constant__ Batch<SplitPlain<T>, NB> zs,
+                                  const __grid_constant__ Batch<St, NB> sts) {
+  typedef typename cplx_t<T>::type C;
+  pdl_begin();
+  const C *Z = zs.f[NB > 1 ? blockIdx.z : 0].B;
+  const St &st = sts.f[NB > 1 ? blockIdx.z : 0];
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (2 * k > n) return;
+  const C zk = Z[k], zm = Z[k == 0 ? 0 : n - k], w = __ldg(&tw2[k]);
+  const T sx = zk.x + zm.x, sy = zk.y - zm.y, dx = zk.x - zm.x, dy = zk.y + zm.y;
+  const T px = fma_t(dx, w.y, fma_t(dy, w.x, sx)), py = fma_t(-dx, w.x, fma_t(dy, w.y, sy));
+  st(0, 0, k, mk<T>((T) 0.5 * px, (T) 0.5 * py));
+  if (2 * k != n) st(0, 0, n - k, mk<T>(fma_t((T) -0.5, px, sx), fma_t((T) 0.5, py, -sy)));
+}
+
+// Functors of the potential's and the propagation's z passes, which split lines
+// serve (kLine1D), and those with the scratch (SpecStoreZ, SpecLoadZ)
+template <class F> __host__ __device__ constexpr auto line_1d_of(int) -> decltype(F::kLine1D, bool()) { return F::kLine1D; }
+template <class F> __host__ __device__ constexpr bool line_1d_of(long) { return false; }
+template <class F> auto scratch_of(const F &f, int) -> decltype(f.scratch) { return f.scratch; }
+template <class F> std::nullptr_t scratch_of(const F &, long) { return nullptr; }
+
+// Returns -1 when the line is not split: more than one line, FP32 (not bound by
+// its operations: one launch is faster than two), shorter than kSplitLine, or
+// no scratch.
+template <typename T, int MODE, int NB, class Ld, class St>
+int split_lines(int n, int na, int nb, int nf, T sign, const Batch<Ld, NB> &ld, const Batch<St, NB> &st) {
+  typedef typename cplx_t<T>::type C;
+  if constexpr (std::is_same<T, double>::value) {
+    if (na * nb != 1 || n < kSplitLine) return -1;
+    C *scr[NB];
+    for (int i = 0; i < nf; i++) {
+      C *a = (C *) scratch_of(ld.f[i], 0), *b = (C *) scratch_of(st.f[i], 0);
+      scr[i] = a ? a : b;
+      if (!scr[i]) return -1;
+    }
+    int n1 = 1;
+    for (int d = 2; d * d <= n; d++)
+      if (n % d == 0) n1 = d;
+    if (n1 < 16) return -1;
+    const int n2 = n / n1;
+    FftPlan<T> p1, p2, pn, pr;
+    DFT_TRY(get_plan<T>(n1, &p1, true));
+    DFT_TRY(get_plan<T>(n2, &p2, true));
+    DFT_TRY(get_plan<T>(n, &pn));
+    if (MODE != LINE_C2C) DFT_TRY(get_plan<T>(2 * n, &pr));
+    const int inv = sign > (T) 0;
+    Batch<SplitMid<T>, NB> mid;
+    memset(&mid, 0, sizeof(mid));
+    // R2C: pass 1 goes to the spectrum's place, pass 2 to the scratch, the third launch back
+    for (int i = 0; i < nf; i++) {
+      C *A = scr[i];
+      if constexpr (MODE == LINE_R2C) A = st.f[i].spec;
+      mid.f[i] = SplitMid<T>{A, pn.tw, n2};
+    }
+    if constexpr (MODE == LINE_C2R) {
+      Batch<SplitPre<T, Ld>, NB> l1;
+      memset(&l1, 0, sizeof(l1));
+      for (int i = 0; i < nf; i++) l1.f[i] = SplitPre<T, Ld>{ld.f[i], pr.tw, n, n2};
+      DFT_TRY((launch_generic_lines<T, LINE_C2C, NB>(p1, nullptr, 1, n2, nf, (T) -1, 0, 0, l1, mid, rt().stream)));
+    } else {
+      Batch<SplitLoad<Ld>, NB> l1;
+      memset(&l1, 0, sizeof(l1));
+      for (int i = 0; i < nf; i++) l1.f[i] = SplitLoad<Ld>{ld.f[i], n2, inv};
+      DFT_TRY((launch_generic_lines<T, LINE_C2C, NB>(p1, nullptr, 1, n2, nf, (T) -1, 0, 0, l1, mid, rt().stream)));
+    }
+    if constexpr (MODE == LINE_R2C) {
+      Batch<SplitPlain<T>, NB> z;
+      Batch<SplitStore<SplitPlain<T>>, NB> s2;
+      memset(&z, 0, sizeof(z));
+      memset(&s2, 0, sizeof(s2));
+      for (int i = 0; i < nf; i++) {
+        z.f[i] = SplitPlain<T>{scr[i]};
+        s2.f[i] = SplitStore<SplitPlain<T>>{z.f[i], n1, 0};
+      }
+      DFT_TRY((launch_generic_lines<T, LINE_C2C, NB>(p2, nullptr, 1, n1, nf, (T) -1, 1, 0, mid, s2, rt().stream)));
+      launch_pdl(split_post_kernel<T, NB, St>, dim3((n / 2 + 64) / 64, 1, nf), 64, 0, rt().stream, n, pr.tw, z, st);
+      DFT_CHECK_LAUNCH();
+    } else {
+      Batch<SplitStore<St>, NB> s2;
+      memset(&s2, 0, sizeof(s2));
+      for (int i = 0; i < nf; i++) s2.f[i] = SplitStore<St>{st.f[i], n1, inv};
+      DFT_TRY((launch_generic_lines<T, LINE_C2C, NB>(p2, nullptr, 1, n1, nf, (T) -1, 1, 0, mid, s2, rt().stream)));
+    }
+    return DFTGPU_OK;
+  }
+  return -1;
+}
+
 // Line passes of nf fields (at most NB) of one shape in one launch.
 // extra_bytes: algorithmic bytes read / written by the fused functors beyond
 // the transformed line data itself (e.g. the potential read by a phase load).
@@ -1002,6 +1140,11 @@ int launch_lines_batch(int n_fft, int na, int nb, int nf, T sign, const Batch<Ld
       }
       if (rc >= 0) return rc;
     }
+  }
+  // only the functor pairs of the transforms with scratch instantiate the split form
+  if constexpr (line_1d_of<Ld>(0) || line_1d_of<St>(0)) {
+    const int rc = split_lines<T, MODE, NB>(n_fft, na, nb, nf, sign, ld, st);
+    if (rc >= 0) return rc;
   }
   FftPlan<T> p1, p2;
   DFT_TRY(get_plan<T>(n_fft, &p1, small_pass(n_fft, na * nf, nb)));

@@ -230,6 +230,7 @@ template <typename T> int k_axpb(T *p, size_t n, T a, T b) {   // p = a p + b
 // any phase factor is formed; PhaseStore prefetches its V lines into L2
 // before the transform, so the loads after it do not wait on DRAM.
 template <typename T> struct PhaseLoad {   // psi * exp(-i V dt / 2)
+  static constexpr bool kLine1D = true;
   typedef typename cplx_t<T>::type C;
   static constexpr bool kSplit = true, kAhead = true;
   struct Raw { C p, v; };
@@ -251,6 +252,7 @@ template <typename T> struct PhaseLoad {   // psi * exp(-i V dt / 2)
   __device__ C operator()(int x, int y, int e) const { return cook(fetch(x, y, e)); }
 };
 template <typename T> struct PhaseStore {
+  static constexpr bool kLine1D = true;
   typedef typename cplx_t<T>::type C;
   static constexpr bool kSplit = true, kBoundedStore = true;
   C *psi; const C *V; int ny, nz; T hr, hi;
@@ -359,7 +361,8 @@ template <typename T> int strang(wf *g, cgrid *dst, cgrid *src, cgrid *V, double
   if (!spec) return DFTGPU_ERR_NOMEM;
   const T hr = (T) (0.5 * dr), hi = (T) (0.5 * di);
   PhaseLoad<T> ld{(const C *) src->value, (const C *) V->value, ny, nz, hr, hi};
-  SpecStoreZ<T> sz{spec, nx, ny};
+  const size_t scr = wf_scratch(src);
+  SpecStoreZ<T> sz{spec, nx, ny, scr ? spec + scr : nullptr};
   DFT_TRY((launch_lines<T, LINE_C2C, 1, 0>(nz, nx, ny, (T) -1, ld, sz)));
   KinArgs<T> K;
   const double m = g->mass;
@@ -368,7 +371,7 @@ template <typename T> int strang(wf *g, cgrid *dst, cgrid *src, cgrid *V, double
               mg->kx0, mg->ky0, mg->kz0, spec);
   K.cn = cn;
   DFT_TRY(kinetic_yxy<T>(K, spec));
-  SpecLoadZ<T> lz{spec, nx, ny};
+  SpecLoadZ<T> lz{spec, nx, ny, scr ? spec + scr : nullptr};
   PhaseStore<T> st{(C *) dst->value, (const C *) V->value, ny, nz, hr, hi};
   return launch_lines<T, LINE_C2C, 0, 1>(nz, nx, ny, (T) 1, lz, st);
 }

@@ -35,9 +35,11 @@ void *dev_alloc(size_t bytes);
 void dev_free(void *p);
 int check_dims(INT nx, INT ny, INT nz);
 
+inline size_t wf_scratch(const cgrid *c) { return c->prec == DFTGPU_FP64 && c->nx == 1 && c->ny == 1 ? gsize(c) : 0; }
 inline void *wf_spec(wf *g) {
   WfPriv *p = (WfPriv *) g->priv;
-  if (!p->spec) p->spec = dev_alloc(gsize(g->grid) * 2 * elem_size(g->grid->prec));
+  const size_t n = gsize(g->grid);   // 1-D FP64: and as much scratch (split lines, fft.cuh)
+  if (!p->spec) p->spec = dev_alloc((wf_scratch(g->grid) ? 2 * n : n) * 2 * elem_size(g->grid->prec));
   return p->spec;
 }
 

@@ -208,6 +208,7 @@ template <typename T> struct SpecStoreZ {           // z pass output
   static constexpr bool kBatch = true;
   static constexpr bool kSpecZ = true;
   typename cplx_t<T>::type *spec; int nx, ny;
+  typename cplx_t<T>::type *scratch = nullptr;      // as many values as the line, for split lines (fft.cuh)
   __device__ void operator()(int x, int y, int k, typename cplx_t<T>::type v) const {
     spec[((size_t) k * nx + x) * ny + y] = v;
   }
@@ -220,6 +221,7 @@ template <typename T> struct SpecLoadZ {            // z pass input (inverse); i
   typedef typename cplx_t<T>::type C;                // run per plane, not prefetched ahead
   static constexpr bool kSpecZ = true;
   const C *spec; int nx, ny;
+  C *scratch = nullptr;                              // as in SpecStoreZ
   __device__ C operator()(int x, int y, int k) const {
     return spec[((size_t) k * nx + x) * ny + y];
   }
@@ -240,6 +242,7 @@ template <typename T> struct SpecLineY {            // y pass in place: line (kz
   }
 };
 template <typename T> struct RealPairLoad {         // packed (f[2e], f[2e+1]) of a real row
+  static constexpr bool kLine1D = true;
   static constexpr bool kBatch = true;
   static constexpr bool kAhead = true;
   const T *f; int ny, nz;
@@ -253,6 +256,7 @@ template <typename T> struct RealPairLoad {         // packed (f[2e], f[2e+1]) o
   }
 };
 template <typename T> struct RealPairStore {        // real row <- scale * (re, im)
+  static constexpr bool kLine1D = true;
   static constexpr bool kBatch = true;
   T *f; int ny, nz; T scale;
   __device__ void operator()(int x, int y, int e, typename cplx_t<T>::type v) const {
@@ -268,6 +272,7 @@ template <typename T> struct RealPairStore {        // real row <- scale * (re, 
 // so without the split every element's psi loads would wait for the previous
 // element's store.
 template <typename T> struct DensityPairLoad {
+  static constexpr bool kLine1D = true;
   typedef typename cplx_t<T>::type C;
   static constexpr bool kAhead = true, kSplit = true;
   struct Raw { C a, b; T *dst; };
@@ -296,6 +301,7 @@ template <typename T> struct DensityPairLoad {
 // applies the predict-correct scale.  Algorithmic bytes beyond a real-row
 // store: P is read and written (3 real fields).
 template <typename T> struct PotAddPairStore {
+  static constexpr bool kLine1D = true;
   typedef typename cplx_t<T>::type C;
   static constexpr bool kSplit = true;
   C *pot; int ny, nz; T scale;
@@ -372,9 +378,10 @@ int irfft_yz(typename cplx_t<T>::type *spec, const St &st, int nx, int ny, int n
 }
 
 // ---------------------------------------------------------------- z passes and convolutions
-// The z passes of nf real fields, up to LINE_BATCH in one launch.
+// The z passes of nf real fields, up to LINE_BATCH in one launch; scr: offset of
+// each spectrum's scratch in its buffer (spec_scratch(), 0: none).
 template <typename T>
-int zpass_fwd_n(const T *const *f, typename cplx_t<T>::type *const *spec, int nf, int nx, int ny, int nz) {
+int zpass_fwd_n(const T *const *f, typename cplx_t<T>::type *const *spec, int nf, int nx, int ny, int nz, size_t scr) {
   for (int i0 = 0; i0 < nf; i0 += LINE_BATCH) {
     const int m = nf - i0 < LINE_BATCH ? nf - i0 : LINE_BATCH;
     Batch<RealPairLoad<T>, LINE_BATCH> ld;
@@ -383,14 +390,14 @@ int zpass_fwd_n(const T *const *f, typename cplx_t<T>::type *const *spec, int nf
     memset(&st, 0, sizeof(st));
     for (int i = 0; i < m; i++) {
       ld.f[i] = RealPairLoad<T>{f[i0 + i], ny, nz};
-      st.f[i] = SpecStoreZ<T>{spec[i0 + i], nx, ny};
+      st.f[i] = SpecStoreZ<T>{spec[i0 + i], nx, ny, scr ? spec[i0 + i] + scr : nullptr};
     }
     DFT_TRY((launch_lines_batch<T, LINE_R2C, 1, 0, LINE_BATCH>(nz / 2, nx, ny, m, (T) -1, ld, st)));
   }
   return DFTGPU_OK;
 }
 template <typename T>
-int zpass_inv_n(typename cplx_t<T>::type *const *spec, T *const *f, int nf, int nx, int ny, int nz) {
+int zpass_inv_n(typename cplx_t<T>::type *const *spec, T *const *f, int nf, int nx, int ny, int nz, size_t scr) {
   for (int i0 = 0; i0 < nf; i0 += LINE_BATCH) {
     const int m = nf - i0 < LINE_BATCH ? nf - i0 : LINE_BATCH;
     Batch<SpecLoadZ<T>, LINE_BATCH> ld;
@@ -398,7 +405,7 @@ int zpass_inv_n(typename cplx_t<T>::type *const *spec, T *const *f, int nf, int 
     memset(&ld, 0, sizeof(ld));
     memset(&st, 0, sizeof(st));
     for (int i = 0; i < m; i++) {
-      ld.f[i] = SpecLoadZ<T>{spec[i0 + i], nx, ny};
+      ld.f[i] = SpecLoadZ<T>{spec[i0 + i], nx, ny, scr ? spec[i0 + i] + scr : nullptr};
       st.f[i] = RealPairStore<T>{f[i0 + i], ny, nz, (T) 1};
     }
     DFT_TRY((launch_lines_batch<T, LINE_C2R, 0, 1, LINE_BATCH>(nz / 2, nx, ny, m, (T) 1, ld, st)));

@@ -24,12 +24,19 @@ struct OtPriv {
 
 void *dev_alloc(size_t bytes);
 
+// Offset of the scratch that follows a half spectrum in its buffer: the FP64
+// lines of 1-D grids are transformed in parts (split lines, fft.cuh).
+inline size_t spec_scratch(int prec, int nx, int ny, int nz) {
+  return prec == DFTGPU_FP64 && nx == 1 && ny == 1 ? (size_t) nz / 2 + 1 : 0;
+}
+
 inline void *ot_real(OtPriv *P, int i) {
   if (!P->real[i]) P->real[i] = dev_alloc((size_t) P->nx * P->ny * P->nz * elem_size(P->prec));
   return P->real[i];
 }
 inline void *ot_spec(OtPriv *P, int i) {
-  if (!P->spec[i]) P->spec[i] = dev_alloc((size_t) (P->nz / 2 + 1) * P->nx * P->ny * 2 * elem_size(P->prec));
+  const size_t n = (size_t) (P->nz / 2 + 1) * P->nx * P->ny;
+  if (!P->spec[i]) P->spec[i] = dev_alloc((spec_scratch(P->prec, P->nx, P->ny, P->nz) ? 2 * n : n) * 2 * elem_size(P->prec));
   return P->spec[i];
 }
 

@@ -43,22 +43,23 @@ template <typename T> struct Fields {
   // y passes to convolve(); with the fused plane passes selected the y passes
   // belong to the transforms.
   static bool yz_fused() { return !fused_zy_off(); }
+  size_t scr() const { return spec_scratch(P->prec, nx, ny, nz); }
   template <class Ld> int zfwd(const Ld &ld, C *spec, double extra_bytes = 0.0) {
     if (yz_fused()) return rfft_zy<T>(ld, spec, nx, ny, nz, extra_bytes);
-    SpecStoreZ<T> st{spec, nx, ny};
+    SpecStoreZ<T> st{spec, nx, ny, scr() ? spec + scr() : nullptr};
     return launch_lines<T, LINE_R2C, 1, 0>(nz / 2, nx, ny, (T) -1, ld, st, extra_bytes);
   }
   template <class St> int zinv(C *spec, const St &st, double extra_bytes = 0.0) {
     if (yz_fused()) return irfft_yz<T>(spec, st, nx, ny, nz, extra_bytes);
-    SpecLoadZ<T> ld{spec, nx, ny};
+    SpecLoadZ<T> ld{spec, nx, ny, scr() ? spec + scr() : nullptr};
     return launch_lines<T, LINE_C2R, 0, 1>(nz / 2, nx, ny, (T) 1, ld, st, extra_bytes);
   }
   int zfwd_n(int n, const T *const *f, C *const *spec) {
-    if (!yz_fused()) return zpass_fwd_n<T>(f, spec, n, nx, ny, nz);
+    if (!yz_fused()) return zpass_fwd_n<T>(f, spec, n, nx, ny, nz, scr());
     return par_for(n, [&](int i) { return fwd(f[i], spec[i]); });
   }
   int zinv_n(int n, C *const *spec, T *const *f) {
-    if (!yz_fused()) return zpass_inv_n<T>(spec, f, n, nx, ny, nz);
+    if (!yz_fused()) return zpass_inv_n<T>(spec, f, n, nx, ny, nz, scr());
     return par_for(n, [&](int i) { return inv(spec[i], f[i]); });
   }
   int conv(XConvArgs<T> &A, unsigned ydone = 0) { return yz_fused() ? launch_xconv<T>(A) : convolve<T>(A, ydone); }
@@ -66,13 +67,13 @@ template <typename T> struct Fields {
   // over several convolutions after their y passes)
   int fwd_n(int n, const T *const *f, C *const *spec) {
     if (yz_fused()) return par_for(n, [&](int i) { return fwd(f[i], spec[i]); });
-    DFT_TRY(zpass_fwd_n<T>(f, spec, n, nx, ny, nz));
+    DFT_TRY(zpass_fwd_n<T>(f, spec, n, nx, ny, nz, scr()));
     return ypass_batch<T>(spec, n, nx, ny, nz / 2 + 1, (T) -1);
   }
   int inv_n(int n, C *const *spec, T *const *f) {
     if (yz_fused()) return par_for(n, [&](int i) { return inv(spec[i], f[i]); });
     DFT_TRY(ypass_batch<T>(spec, n, nx, ny, nz / 2 + 1, (T) 1));
-    return zpass_inv_n<T>(spec, f, n, nx, ny, nz);
+    return zpass_inv_n<T>(spec, f, n, nx, ny, nz, scr());
   }
   int inv(C *spec, T *f) {
     RealPairStore<T> st{f, ny, nz, (T) 1};

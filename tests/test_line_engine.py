@@ -107,3 +107,51 @@ def test_convolutions(shape, prec):
     ref = np.roll(out[0], shift, axis=(0, 1, 2))
     # the terms of the potential are up to 1e3 times its own size at this noise
     assert np.linalg.norm(out[1] - ref) <= 1e3 * 4 * eps(prec) * np.log2(psi.size) * np.linalg.norm(ref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("shape", [(1, 1, 500), (1, 1, 512), (1, 1, 1000), (1, 1, 1024), (1, 1, 2160), (1, 1, 4096), (2, 2, 1024)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_long_lines(shape, prec):
+    """Lines around the length from which a 1-D grid's line is transformed in parts: plain potential
+    V = LJ*rho + c2/2 rb^2 + c3/3 rb^3 + w*((c2 rb + c3 rb^2) rho), rb = w*rho, from the library's own kernel spectra
+    with numpy's transforms, and one complex step there and back.  The four convolutions' terms are up to a few
+    times the potential: 16 eps log2 N; a step forwards and backwards: two propagations' tolerance."""
+    import libdft_gb300 as G
+    G.check(G.lib().dftgpu_init(0), "init")
+    G.set_precision(prec)
+    h = 0.4
+    rng = np.random.default_rng(11)
+    psi = np.sqrt(0.00323) * (1 + 0.05 * rng.standard_normal(shape)) * np.exp(0.3j * rng.standard_normal(shape))
+    if prec:
+        psi = psi.astype(np.complex64).astype(np.complex128)
+    try:
+        w = G.Wf(shape, h)
+        ot = G.OT(G.DFT_OT_PLAIN, w)
+        P = G.CGrid(shape, h)
+        w.set(psi)
+        P.zero()
+        ot.potential(P, w)
+        got = P.get().real
+        ker = [ot.kernel(k) for k in (0, 1)]
+        c2, c3 = ot.params.c2, ot.params.c3
+        P.zero()
+        w.propagate(P, 9.0 + 0j)
+        w.propagate(P, -9.0 + 0j)
+        back = w.get()
+        for x in (P, ot, w):
+            x.free()
+    finally:
+        G.set_precision(G.FP64)
+    nx, ny, nz = shape
+    ix, iy = np.minimum(np.arange(nx), nx - np.arange(nx)), np.minimum(np.arange(ny), ny - np.arange(ny))
+    full = [np.transpose(k[:, ix][:, :, iy], (1, 2, 0)) for k in ker]      # [kx][ky][kz], scaled by step^3 / N
+    def conv(k, f):
+        return np.fft.irfftn(k * np.fft.rfftn(f), s=shape, axes=(0, 1, 2)) * f.size
+    rho = np.abs(psi) ** 2
+    rb = conv(full[1], rho)
+    ref = conv(full[0], rho) + c2 / 2 * rb ** 2 + c3 / 3 * rb ** 3 + conv(full[1], (c2 * rb + c3 * rb ** 2) * rho)
+    e = eps(prec) * np.log2(psi.size)
+    assert np.linalg.norm(got - ref) <= 16 * e * np.linalg.norm(ref)
+    assert np.linalg.norm(back - psi) <= 2 * (8 * e + 16 * eps(prec)) * np.linalg.norm(psi)
