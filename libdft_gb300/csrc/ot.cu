@@ -437,7 +437,7 @@ template <typename T> static int potential_t(dft_ot_functional *otf, cgrid *Pg, 
                         3.0 * nb, "ot_thermal"));
   }
 
-  // forward transforms of the produced fields (independent: parallel branches)
+  // forward z passes of the produced fields
   {
     const T *in[8]; C *sp[8]; int n = 0;
     if (loc) { in[n] = r[R_Q]; sp[n++] = s[9]; }
