@@ -57,22 +57,49 @@ int bad_arg(const char *what) { set_error(DFTGPU_ERR_ARG, "%s", what); return DF
     if (!(cond)) { bad_arg(what ": NULL argument"); return __VA_ARGS__; } \
   } while (0)
 
+// What a captured step was formed from on the host: its kernels hold the
+// objects' public fields (functional parameters, mass, target norm,
+// propagator, momentum, data pointers) by value, and a caller may set any of
+// them between two calls.
+struct StepKey {
+  dft_ot_functional *otf;
+  wf *g, *gp;
+  cgrid *P;
+  rgrid *vext;
+  cudaStream_t user;
+  double mu0, dr, di;
+  int renorm;
+  dft_ot_functional functional;
+  wf wave, predicted;
+  cgrid wave_grid, predicted_grid, potential;
+  rgrid external, density;
+};
+void step_key(StepKey &k, dft_ot_functional *otf, wf *g, wf *gp, cgrid *P, rgrid *vext, double mu0, double dr, double di,
+              int renorm) {
+  memset(&k, 0, sizeof(k));   // padding too: keys are compared as bytes
+  k.otf = otf; k.g = g; k.gp = gp; k.P = P; k.vext = vext; k.user = rt().stream;
+  k.mu0 = mu0; k.dr = dr; k.di = di; k.renorm = renorm;
+  memcpy(&k.functional, otf, sizeof(k.functional));
+  memcpy(&k.wave, g, sizeof(k.wave));
+  memcpy(&k.predicted, gp, sizeof(k.predicted));
+  memcpy(&k.wave_grid, g->grid, sizeof(k.wave_grid));
+  memcpy(&k.predicted_grid, gp->grid, sizeof(k.predicted_grid));
+  memcpy(&k.potential, P, sizeof(k.potential));
+  if (vext) memcpy(&k.external, vext, sizeof(k.external));
+  if (otf->density) memcpy(&k.density, otf->density, sizeof(k.density));
+}
+
 // Instantiated graph of one predict-correct step, replayed by dftgpu_run when
-// it is called again with the same arguments.  Any free of a grid, wave
-// function or functional bumps g_generation and so invalidates it.
+// it is called again with the same arguments and nothing that the step was
+// formed from has changed.  Any free of a grid, wave function or functional
+// bumps g_generation and so invalidates it.
 unsigned long g_generation = 1;
 struct GraphCache {
   cudaGraphExec_t exec = nullptr;
-  cudaStream_t cap = nullptr, user = nullptr;
+  cudaStream_t cap = nullptr;
   cudaEvent_t ev = nullptr;
   unsigned long gen = 0;
-  dft_ot_functional *otf = nullptr;
-  wf *g = nullptr, *gp = nullptr;
-  cgrid *P = nullptr;
-  rgrid *vext = nullptr;
-  double mu0 = 0, dr = 0, di = 0;
-  double k0[3] = { 0, 0, 0 };   // moving-background momentum captured in the kinetic passes
-  int renorm = 0;
+  StepKey key;
 } g_graph;
 
 }  // namespace
@@ -881,10 +908,9 @@ int dftgpu_run(dft_ot_functional *otf, wf *gwf, wf *gwfp, cgrid *P, rgrid *vext,
     return DFTGPU_OK;
   }
   GraphCache &G = g_graph;
-  const bool hit = G.exec && G.gen == g_generation && G.otf == otf && G.g == gwf && G.gp == gwfp && G.P == P &&
-                   G.vext == vext && G.mu0 == mu0 && G.dr == dr && G.di == di && G.renorm == renorm &&
-                   G.user == rt().stream && G.k0[0] == gwf->grid->kx0 && G.k0[1] == gwf->grid->ky0 &&
-                   G.k0[2] == gwf->grid->kz0;
+  StepKey key;
+  step_key(key, otf, gwf, gwfp, P, vext, mu0, dr, di, renorm);
+  const bool hit = G.exec && G.gen == g_generation && memcmp(&key, &G.key, sizeof(key)) == 0;
   if (!hit) {
     // one step eagerly: allocates work buffers and FFT tables outside capture
     DFT_TRY(step_with_renorm(otf, gwf, gwfp, P, vext, mu0, dr, di, renorm));
@@ -914,9 +940,8 @@ int dftgpu_run(dft_ot_functional *otf, wf *gwf, wf *gwfp, cgrid *P, rgrid *vext,
     }
     if (graph) cudaGraphDestroy(graph);
     if (!rc) {
-      G.gen = g_generation; G.otf = otf; G.g = gwf; G.gp = gwfp; G.P = P; G.vext = vext;
-      G.mu0 = mu0; G.dr = dr; G.di = di; G.renorm = renorm; G.user = user;
-      G.k0[0] = gwf->grid->kx0; G.k0[1] = gwf->grid->ky0; G.k0[2] = gwf->grid->kz0;
+      G.gen = g_generation;
+      memcpy(&G.key, &key, sizeof(key));
     }
   }
   for (INT s = 0; !rc && s < nsteps; s++)
