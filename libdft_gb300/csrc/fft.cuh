@@ -226,7 +226,12 @@ __device__ __forceinline__ void small_dft(C *u, T s) {
 // product by the twiddle followed by the sums takes eight, with two roundings
 // on the way to each output instead of three (t.x c is Re(z b) to one
 // rounding whatever the size of r).  FP32 is not bound by its operations and
-// keeps (cos, sin) pairs rounded to the unit circle.
+// keeps (cos, sin) pairs rounded to the unit circle.  Its untwiddled constants
+// scale the norm by a fixed amount a transform (1/sqrt(2) and the pair of
+// pi/8 are below the circle, radix 5 above it): with every c1 as it rounds
+// radix 16 lowers it by 2.7e-8, with one of the four rounded up by 2.0e-8,
+// which brings lengths 240, 160 and 80 from -2.1e-8, -9.1e-9 and -5.3e-9 to
+// -1.3e-8, -2.3e-9 and 1e-9 (all four up: 80 and 160 at +2e-8).
 __device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
 
@@ -302,8 +307,8 @@ __device__ __forceinline__ void poly_eval(const C *u, C *y, const PolyTw<R, C> &
         else if (8 * j == 3 * M) bf_8th<1>(e[j], o[j]);
         else {             // M = 16, odd j: exp(-2 pi i j / 16)
           C z;
-          if constexpr (sizeof(e[0].x) == 4) {   // (cos, sin)
-            if (j == 1 || j == 5) { z.x = ff::FF_C1; z.y = -ff::FF_S1; } else { z.x = ff::FF_S1; z.y = -ff::FF_C1; }
+          if constexpr (sizeof(e[0].x) == 4) {   // (cos, sin); one of the four c1 rounded up (below)
+            if (j == 1 || j == 5) { z.x = j == 1 ? ff::FF_C1B : ff::FF_C1; z.y = -ff::FF_S1; } else { z.x = ff::FF_S1; z.y = -ff::FF_C1; }
           } else {                               // (cos, tan) of -pi/8 and -3 pi/8: tan(pi/8) = sqrt(2) - 1
             if (j == 1 || j == 5) { z.x = 0.923879532511286756128; z.y = -0.414213562373095048802; }
             else { z.x = 0.382683432365089771728; z.y = -2.414213562373095048802; }
