@@ -56,26 +56,31 @@ int factorize_fp64(int n, int cap, int *radix, int *nst) {
   search(n, cap, 0, 0.0, 0, cur, &best, radix, nst);
   return best < 1e9 ? DFTGPU_OK : DFTGPU_ERR_SIZE;
 }
-// FP32: few stages, not bound by operations (16 first: 240^3 12.0 ms in two steps against 13.0 as 15, 16)
+// FP32 is not bound by operations: few stages, 16 or 8 first (its first stage
+// has no twiddles).  One propagation, us, this order / the odd radices first:
+// 240^3 457 / 495, 120^3 84 / 87, 360 x 360 x 180 963 / 1018; rms error of a
+// round trip at 120^3 2.17e-7 / 2.29e-7.  A 2 left alone beside a 16: 8 x 4 has
+// as many butterflies in both stages (288^3 1173 / 1245 as 16, 9, 2; twenty
+// steps of 64^3, z half 32, 2391 / 2475).  A 16 alone stays one stage: 4 x 4
+// takes 3 of 24 us off a propagation of 16^3, at 3 % more rms error.
 int factorize_fp32(int n, int *radix, int *nst) {
   int m = n, k = 0, a = 0, b = 0, c = 0;
-  // short lines: as many butterflies in both stages (64^3 plain, z half 32: 2391 us for
-  // twenty steps against 2475 as 16, 2; potential 16 x 16 x 32 80 against 84 as one radix-16 stage)
-  if (n == 32) { radix[0] = 8; radix[1] = 4; *nst = 2; return DFTGPU_OK; }
-  if (n == 16) { radix[0] = 4; radix[1] = 4; *nst = 2; return DFTGPU_OK; }
   while (m % 2 == 0) { m /= 2; a++; }
   while (m % 3 == 0) { m /= 3; b++; }
   while (m % 5 == 0) { m /= 5; c++; }
   if (m != 1) return DFTGPU_ERR_SIZE;
-  // few stages: radix 16 for the power of two, one 8 / 4 / 2 for its rest;
-  // 15 = 3 x 5 and 9 = 3 x 3 for the odd part; a rest of 2 or 4 merged with
-  // a rest of 3 (6, 12) or 2 with a 5 (10)
+  // radix 16 for the power of two, one 8 / 4 / 2 for its rest; 15 = 3 x 5 and
+  // 9 = 3 x 3 for the odd part; a rest of 2 or 4 merged with a rest of 3 (6,
+  // 12) or 2 with a 5 (10), a 2 that stays alone beside a 16 as 8 x 4
   while (a >= 4) { radix[k++] = 16; a -= 4; }
+  const int n16 = k;
   int r2 = 1 << a;
+  if (r2 == 8 && n16 == 0) { radix[k++] = 8; r2 = 1; }
   while (b >= 1 && c >= 1) { radix[k++] = 15; b--; c--; }
   while (b >= 2) { radix[k++] = 9; b -= 2; }
   if ((r2 == 2 || r2 == 4) && b == 1) { radix[k++] = 3 * r2; r2 = 1; b = 0; }
   else if (r2 == 2 && c >= 1) { radix[k++] = 10; r2 = 1; c--; }
+  if (r2 == 2 && n16 > 0) { radix[n16 - 1] = 8; r2 = 4; }
   if (r2 > 1) radix[k++] = r2;
   if (b == 1) radix[k++] = 3;
   while (c-- > 0) radix[k++] = 5;
