@@ -57,9 +57,9 @@ int factorize_fp64(int n, int cap, int *radix, int *nst) {
   return best < 1e9 ? DFTGPU_OK : DFTGPU_ERR_SIZE;
 }
 // FP32 is not bound by operations: few stages, 16 or 8 first (its first stage
-// has no twiddles).  One propagation, us, this order / the odd radices first:
-// 240^3 457 / 495, 120^3 84 / 87, 360 x 360 x 180 963 / 1018; rms error of a
-// round trip at 120^3 2.17e-7 / 2.29e-7.  A 2 left alone beside a 16: 8 x 4 has
+// has no twiddles): two steps of 240^3 12.0 ms as 16, 15 and 13.0 as 15, 16;
+// one propagation of 120^3 84 us as 8, 15 and 87 as 15, 8, with rms errors of
+// 2.17e-7 and 2.29e-7.  A 2 left alone beside a 16: 8 x 4 has
 // as many butterflies in both stages (288^3 1173 / 1245 as 16, 9, 2; twenty
 // steps of 64^3, z half 32, 2391 / 2475).  A 16 alone stays one stage: 4 x 4
 // takes 3 of 24 us off a propagation of 16^3, at 3 % more rms error.
@@ -161,15 +161,19 @@ template <typename T> int get_plan(int n, FftPlan<T> *plan, bool small) {
 template int get_plan<float>(int, FftPlan<float> *, bool);
 template int get_plan<double>(int, FftPlan<double> *, bool);
 
-size_t max_smem() {
-  static size_t v = 0;
-  if (!v) {
-    int dev = 0, m = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess &&
-        cudaDeviceGetAttribute(&m, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess)
-      v = (size_t) m;
+const DevLimits &dev_limits() {
+  static DevLimits known[64];
+  static std::mutex mu;
+  static const DevLimits none = { -1, 0 };
+  int dev = 0, smem = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return none;
+  std::lock_guard<std::mutex> lock(mu);
+  DevLimits &d = known[dev];
+  if (!d.smem && cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess) {
+    d.id = dev;
+    d.smem = (size_t) smem;
   }
-  return v;
+  return d.smem ? d : none;
 }
 
 // About 16 values per thread (one butterfly of radix 16) at 128 threads in
@@ -178,8 +182,7 @@ size_t max_smem() {
 // FP64 to one full warp of butterflies (an FP64 warp instruction takes its 16 clocks
 // of the SM's pipe whatever the number of its active lanes).
 int choose_tile(int n, int big, int na, int nb, size_t cplx_bytes, int nbufs, bool strided, size_t table, TileShape *t) {
-  const size_t hard = max_smem();
-
+  const size_t hard = dev_limits().smem;
   const int most = cplx_bytes == 16 ? 2560 : 5120;
   int least = strided ? (int) (64 / cplx_bytes) : 1;
   while (cplx_bytes == 16 && least < 32 && least * n < 32 * big) least *= 2;   // a full warp of the largest butterflies
@@ -439,11 +442,7 @@ template <typename T> int launch_xconv(XConvArgs<T> &A) {
   DFT_TRY(choose_tile(A.nx, max_radix(A.plan), A.split ? A.nkz * A.nout : A.nkz, A.ny, sizeof(C), xconv_bufs(A.plan.nst, A.acc_buf), true, 0, &t));
   A.B = t.B;
   A.logB = t.logB;
-  static bool attr = false;
-  if (!attr) {
-    DFT_CUDA(cudaFuncSetAttribute(xconv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) max_smem()));
-    attr = true;
-  }
+  DFT_TRY(smem_opt_in<SmemOptIn<XConvArgs<T> (*)()>>(xconv_kernel<T>));
   launch_pdl(xconv_kernel<T>, dim3((A.ny + t.B - 1) / t.B, A.nkz, A.split ? A.nout : 1), t.threads, t.smem, rt().stream, A);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;

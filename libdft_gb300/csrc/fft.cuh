@@ -25,6 +25,8 @@
 
 #include <type_traits>
 
+#include <atomic>
+
 #include "common.cuh"
 #include "fast_fft.cuh"
 
@@ -801,7 +803,10 @@ template <typename T> inline int max_radix(const FftPlan<T> &p) {
   for (int i = 0; i < p.nst; i++) r = p.radix[i] > r ? p.radix[i] : r;
   return r;
 }
-size_t max_smem();   // opt-in shared memory of the device
+// Limits of the current device, looked up once for each: the allocation-free
+// step serves whichever device is current.  id -1: none.
+struct DevLimits { int id; size_t smem; };   // smem: opt-in shared memory of a CTA
+const DevLimits &dev_limits();
 int choose_tile(int n, int big, int na, int nb, size_t cplx_bytes, int nbufs, bool strided, size_t table, TileShape *t);
 inline int line_bufs(int mode, int nst) { return mode == LINE_C2C ? (nst >= 3 ? 2 : 1) : 2; }
 
@@ -812,13 +817,22 @@ template <typename T, int MODE, int NB, class Ld, class St>
 int launch_generic_lines(const FftPlan<T> &plan, const typename cplx_t<T>::type *tw2, int na, int nb, int nf, T sign,
                          int ef, int efs, const Batch<Ld, NB> &ld, const Batch<St, NB> &st, cudaStream_t stream);
 
-// "Opt-in shared memory already requested" flag per kernel instantiation.
+// "Opt-in shared memory already requested" per kernel instantiation, one bit a
+// device (the attribute belongs to the device's copy of the kernel).
 // It lives in an anonymous namespace so that every translation unit keeps its
 // own flag: without relocatable device code each translation unit registers
 // its own copy of a template kernel, and the attribute must be set on each.
 namespace {
-template <class Kernel> struct SmemOptIn { static bool done; };
-template <class Kernel> bool SmemOptIn<Kernel>::done = false;
+template <class Kernel> struct SmemOptIn { static std::atomic<unsigned long long> done; };
+template <class Kernel> std::atomic<unsigned long long> SmemOptIn<Kernel>::done{0};
+template <class Flag, class K> int smem_opt_in(K kernel) {
+  const DevLimits &d = dev_limits();
+  if (d.id >= 0 && !(Flag::done.load() >> d.id & 1)) {
+    DFT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) d.smem));
+    Flag::done |= 1ull << d.id;
+  }
+  return DFTGPU_OK;
+}
 }  // namespace
 
 bool generic_fft_only();   // DFTGPU_GENERIC_FFT=1 disables the register kernels
@@ -971,10 +985,7 @@ int launch_generic_lines(const FftPlan<T> &plan, const typename cplx_t<T>::type 
   args.logB = t.logB;
   auto kfn = line_fft_kernel<T, MODE, NB, Ld, St>;
   typedef SmemOptIn<LineArgs<T> (*)(Ld *, St *, int (*)[MODE + 1], int (*)[NB])> Flag;
-  if (t.smem > 48 * 1024 && !Flag::done) {
-    DFT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) max_smem()));
-    Flag::done = true;
-  }
+  if (t.smem > 48 * 1024) DFT_TRY(smem_opt_in<Flag>(kfn));
   launch_pdl(kfn, dim3((nb + t.B - 1) / t.B, na, nf), t.threads, t.smem, stream, args, ld, st);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
@@ -1181,11 +1192,7 @@ template <typename T> int launch_generic_xkinetic(KinArgs<T> &A, cudaStream_t st
   A.B = t.B;
   A.logB = t.logB;
   auto kfn = xkinetic_kernel<T>;
-  typedef SmemOptIn<KinArgs<T> (*)()> Flag;
-  if (!Flag::done) {
-    DFT_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) max_smem()));
-    Flag::done = true;
-  }
+  if (t.smem > 48 * 1024) DFT_TRY(smem_opt_in<SmemOptIn<KinArgs<T> (*)()>>(kfn));
   launch_pdl(kfn, dim3((A.ny + t.B - 1) / t.B, A.nkz), t.threads, t.smem, stream, A);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;

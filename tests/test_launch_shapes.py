@@ -1,0 +1,68 @@
+"""The launch code of the library on the CPU: a stand-in for the CUDA runtime
+(tests/cuda/fake_cudart.c) is loaded in front of it in a child process and
+records what would have been launched."""
+import json
+import os
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+from conftest import ROOT
+
+PRELUDE = r"""
+import ctypes as C, json, sys
+fake = C.CDLL(sys.argv[1], mode=C.RTLD_GLOBAL)     # its symbols are found before the CUDA runtime's
+sys.path.insert(0, sys.argv[2])
+import libdft_gb300 as G
+KEYS = ("gx", "gy", "gz", "bx", "by", "bz", "smem", "device", "granted", "programmatic", "func")
+def launches():
+    out = (C.c_long * 11)()
+    r = []
+    for i in range(fake.fake_launches()):
+        fake.fake_launch(i, out)
+        r.append(dict(zip(KEYS, out)))
+    fake.fake_reset()
+    return r
+def noalloc(shape, prec):
+    L = G.lib()
+    p = C.c_void_p(1 << 40)
+    rc = L.dftgpu_wf_propagate_noalloc(p, p, p, *shape, 0.8, G.HELIUM_MASS, 1.0, 0.0, prec, None)
+    assert rc == 0, L.dftgpu_last_error_message()
+    return launches()
+result = {}
+"""
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
+    so = str(tmp_path_factory.mktemp("fake") / "libfake_cudart.so")
+    subprocess.run([os.environ.get("CC", "gcc"), "-O1", "-shared", "-fPIC", "-I", include,
+                    os.path.join(ROOT, "tests", "cuda", "fake_cudart.c"), "-o", so], check=True)
+
+    def go(body):
+        r = subprocess.run([sys.executable, "-c", PRELUDE + body + "\nprint(json.dumps(result))", so, ROOT],
+                           capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-2000:]
+        return json.loads(r.stdout.splitlines()[-1])
+    return go
+
+
+def test_allocation_free_step_on_a_second_device(run):
+    """The allocation-free step serves whichever device is current: a kernel that needs more than 48 KB of shared memory
+    has been granted it on that device, also when another device was used first."""
+    r = run("""
+for shape, prec in (((128, 128, 128), 0), ((1, 1, 4096), 0), ((16, 1000, 24), 1)):
+    for device in (0, 1):
+        fake.fake_set_device(device)
+        result["%s %d" % (shape, device)] = noalloc(shape, prec)
+""")
+    big = 0
+    for case, launches in r.items():
+        assert len(launches) == 5, (case, len(launches))
+        big += sum(l["smem"] > 48 * 1024 for l in launches)
+        assert all(l["granted"] for l in launches), (case, [l for l in launches if not l["granted"]])
+    assert big >= 4   # the cases do reach it, on both devices
