@@ -164,13 +164,15 @@ template int get_plan<double>(int, FftPlan<double> *, bool);
 const DevLimits &dev_limits() {
   static DevLimits known[64];
   static std::mutex mu;
-  static const DevLimits none = { -1, 0 };
-  int dev = 0, smem = 0;
+  static const DevLimits none = { -1, 0, 0 };
+  int dev = 0, smem = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return none;
   std::lock_guard<std::mutex> lock(mu);
   DevLimits &d = known[dev];
-  if (!d.smem && cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess) {
+  if (!d.smem && cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) {
     d.id = dev;
+    d.sms = sms;
     d.smem = (size_t) smem;
   }
   return d.smem ? d : none;
@@ -182,7 +184,8 @@ const DevLimits &dev_limits() {
 // FP64 to one full warp of butterflies (an FP64 warp instruction takes its 16 clocks
 // of the SM's pipe whatever the number of its active lanes).
 int choose_tile(int n, int big, int na, int nb, size_t cplx_bytes, int nbufs, bool strided, size_t table, TileShape *t) {
-  const size_t hard = dev_limits().smem;
+  const DevLimits &dev = dev_limits();
+  const size_t hard = dev.smem;
   const int most = cplx_bytes == 16 ? 2560 : 5120;
   int least = strided ? (int) (64 / cplx_bytes) : 1;
   while (cplx_bytes == 16 && least < 32 && least * n < 32 * big) least *= 2;   // a full warp of the largest butterflies
@@ -190,7 +193,7 @@ int choose_tile(int n, int big, int na, int nb, size_t cplx_bytes, int nbufs, bo
   while (B > 1 && (B * n > most || B >= 2 * nb)) B >>= 1;
   if (B < least) B = least;
   while (B > 1 && B >= 2 * nb) B >>= 1;
-  while (B > least && (size_t) na * ((nb + B - 1) / B) < (size_t) 4 * rt().num_sms) B >>= 1;
+  while (B > least && (size_t) na * ((nb + B - 1) / B) < (size_t) 4 * dev.sms) B >>= 1;
   auto need = [&](int b) { return (size_t) nbufs * b * Tile::pitch(n) * cplx_bytes + table + (table ? (size_t) b * cplx_bytes : 0); };
   while (B > 1 && need(B) > hard) B >>= 1;
   if (need(B) > hard) {

@@ -804,8 +804,8 @@ template <typename T> inline int max_radix(const FftPlan<T> &p) {
   return r;
 }
 // Limits of the current device, looked up once for each: the allocation-free
-// step serves whichever device is current.  id -1: none.
-struct DevLimits { int id; size_t smem; };   // smem: opt-in shared memory of a CTA
+// step serves whichever device is current, also without dftgpu_init.  id -1: none.
+struct DevLimits { int id, sms; size_t smem; };   // smem: opt-in shared memory of a CTA
 const DevLimits &dev_limits();
 int choose_tile(int n, int big, int na, int nb, size_t cplx_bytes, int nbufs, bool strided, size_t table, TileShape *t);
 inline int line_bufs(int mode, int nst) { return mode == LINE_C2C ? (nst >= 3 ? 2 : 1) : 2; }

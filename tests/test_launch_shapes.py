@@ -66,3 +66,17 @@ for shape, prec in (((128, 128, 128), 0), ((1, 1, 4096), 0), ((16, 1000, 24), 1)
         big += sum(l["smem"] > 48 * 1024 for l in launches)
         assert all(l["granted"] for l in launches), (case, [l for l in launches if not l["granted"]])
     assert big >= 4   # the cases do reach it, on both devices
+
+
+def test_allocation_free_step_without_init(run):
+    """The allocation-free step does not need dftgpu_init: its launches are the same before and after it, and small grids
+    spread over every SM (four CTAs each where a CTA keeps its least number of lines)."""
+    r = run("""
+cases = [((64, 64, 64), 0), ((64, 64, 64), 1), ((32, 48, 40), 0)]
+result["before"] = [noalloc(*c) for c in cases]
+G.check(G.lib().dftgpu_init(0), "init")
+fake.fake_reset()
+result["after"] = [noalloc(*c) for c in cases]
+""")
+    assert r["before"] == r["after"]
+    assert all(l["gx"] * l["gy"] >= 4 * 152 for l in r["before"][0])
