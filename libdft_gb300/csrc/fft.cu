@@ -182,8 +182,14 @@ const DevLimits &dev_limits() {
 // FP64 and 256 in FP32; fewer lines per CTA while the launch would not give
 // every SM four CTAs, down to runs of 64 bytes where a side is strided and in
 // FP64 to one full warp of butterflies (an FP64 warp instruction takes its 16 clocks
-// of the SM's pipe whatever the number of its active lanes).
-int choose_tile(int n, int big, int na, int nb, size_t cplx_bytes, int nbufs, bool strided, size_t table, TileShape *t) {
+// of the SM's pipe whatever the number of its active lanes).  Fewer also while
+// `ctas` of them do not fit into an SM's shared memory: three for the line and
+// convolution passes, as many as their registers allow, two for the kinetic
+// pass.  Full potential, us, one / two / three CTAs at least: FP32 288 x 256 x
+// 256 3795 / 2901 / 2900, 320^3 9043 / 7333 / 6875, FP64 288^3 52360 / 44870 /
+// 42910 (four: FP64 216^3 22080 against 21430); FP32 propagation, two / three
+// in the kinetic pass: 288 x 256 x 256 405 / 424, 320^3 1355 / 1379.
+int choose_tile(int n, int big, int na, int nb, size_t cplx_bytes, int nbufs, bool strided, size_t table, int ctas, TileShape *t) {
   const DevLimits &dev = dev_limits();
   const size_t hard = dev.smem;
   const int most = cplx_bytes == 16 ? 2560 : 5120;
@@ -195,6 +201,7 @@ int choose_tile(int n, int big, int na, int nb, size_t cplx_bytes, int nbufs, bo
   while (B > 1 && B >= 2 * nb) B >>= 1;
   while (B > least && (size_t) na * ((nb + B - 1) / B) < (size_t) 4 * dev.sms) B >>= 1;
   auto need = [&](int b) { return (size_t) nbufs * b * Tile::pitch(n) * cplx_bytes + table + (table ? (size_t) b * cplx_bytes : 0); };
+  while (B > least && ctas * (need(B) + 1024) > hard + 1024) B >>= 1;   // 1 KB of an SM's is the system's for each
   while (B > 1 && need(B) > hard) B >>= 1;
   if (need(B) > hard) {
     set_error(DFTGPU_ERR_SIZE, "FFT tile for n=%d does not fit in shared memory", n);
@@ -442,7 +449,7 @@ template <typename T> int launch_xconv(XConvArgs<T> &A) {
     return DFTGPU_OK;
   }
   TileShape t;
-  DFT_TRY(choose_tile(A.nx, max_radix(A.plan), A.split ? A.nkz * A.nout : A.nkz, A.ny, sizeof(C), xconv_bufs(A.plan.nst, A.acc_buf), true, 0, &t));
+  DFT_TRY(choose_tile(A.nx, max_radix(A.plan), A.split ? A.nkz * A.nout : A.nkz, A.ny, sizeof(C), xconv_bufs(A.plan.nst, A.acc_buf), true, 0, 3, &t));
   A.B = t.B;
   A.logB = t.logB;
   DFT_TRY(smem_opt_in<SmemOptIn<XConvArgs<T> (*)()>>(xconv_kernel<T>));

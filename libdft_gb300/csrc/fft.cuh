@@ -796,7 +796,8 @@ __global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 3 : 2) xkinetic_
 // ------------------------------------------------------------ launch helpers
 // Tile of the generic line kernels for lines of length n (largest radix big), nb
 // adjacent lines in each of na planes: lines per CTA, threads and shared memory.  strided: one
-// side's fast index is the line.
+// side's fast index is the line; ctas: CTAs that fit into an SM together, while
+// the tile can be cut.
 struct TileShape { int B, logB, threads; size_t smem; };
 template <typename T> inline int max_radix(const FftPlan<T> &p) {
   int r = 1;
@@ -807,7 +808,7 @@ template <typename T> inline int max_radix(const FftPlan<T> &p) {
 // step serves whichever device is current, also without dftgpu_init.  id -1: none.
 struct DevLimits { int id, sms; size_t smem; };   // smem: opt-in shared memory of a CTA
 const DevLimits &dev_limits();
-int choose_tile(int n, int big, int na, int nb, size_t cplx_bytes, int nbufs, bool strided, size_t table, TileShape *t);
+int choose_tile(int n, int big, int na, int nb, size_t cplx_bytes, int nbufs, bool strided, size_t table, int ctas, TileShape *t);
 inline int line_bufs(int mode, int nst) { return mode == LINE_C2C ? (nst >= 3 ? 2 : 1) : 2; }
 
 constexpr double kBatchBytes = 48e6;   // FP32 spectra of one launch: less than half of L2
@@ -980,7 +981,7 @@ int launch_generic_lines(const FftPlan<T> &plan, const typename cplx_t<T>::type 
   args.e_fast = ef;
   args.e_fast_store = efs;
   TileShape t;
-  DFT_TRY(choose_tile(plan.n, max_radix(plan), na * nf, nb, sizeof(C), line_bufs(MODE, plan.nst), !ef || !efs, 0, &t));
+  DFT_TRY(choose_tile(plan.n, max_radix(plan), na * nf, nb, sizeof(C), line_bufs(MODE, plan.nst), !ef || !efs, 0, 3, &t));
   args.B = t.B;
   args.logB = t.logB;
   auto kfn = line_fft_kernel<T, MODE, NB, Ld, St>;
@@ -1188,7 +1189,7 @@ template <typename T> int launch_xkinetic(KinArgs<T> &A);
 template <typename T> int launch_generic_xkinetic(KinArgs<T> &A, cudaStream_t stream) {
   typedef typename cplx_t<T>::type C;
   TileShape t;
-  DFT_TRY(choose_tile(A.nx, max_radix(A.plan), A.nkz, A.ny, sizeof(C), 2, true, (size_t) A.nx * sizeof(C), &t));
+  DFT_TRY(choose_tile(A.nx, max_radix(A.plan), A.nkz, A.ny, sizeof(C), 2, true, (size_t) A.nx * sizeof(C), 2, &t));
   A.B = t.B;
   A.logB = t.logB;
   auto kfn = xkinetic_kernel<T>;

@@ -80,3 +80,27 @@ result["after"] = [noalloc(*c) for c in cases]
 """)
     assert r["before"] == r["after"]
     assert all(l["gx"] * l["gy"] >= 4 * 152 for l in r["before"][0])
+
+
+def test_tiles_leave_room_for_three_ctas(run):
+    """A tile that can be cut without giving up its runs of 64 bytes (or its FP64 warp of butterflies) lets three CTAs of
+    a line or convolution pass, or two of the kinetic pass, share an SM's 228 KB."""
+    r = run("""
+class Shape(C.Structure):
+    _fields_ = [("B", C.c_int), ("logB", C.c_int), ("threads", C.c_int), ("smem", C.c_size_t)]
+f = G.lib()._ZN6dftgpu11choose_tileEiiiimibmiPNS_9TileShapeE
+f.argtypes = [C.c_int] * 4 + [C.c_size_t, C.c_int, C.c_bool, C.c_size_t, C.c_int, C.POINTER(Shape)]
+result["tiles"] = []
+for cplx in (8, 16):
+    for n in sorted(2 ** a * 3 ** b * 5 ** c for a in range(11) for b in range(7) for c in range(5) if 2 ** a * 3 ** b * 5 ** c <= 1024):
+        for bufs in (1, 2, 3, 4):
+            for ctas in (2, 3):
+                t = Shape()
+                assert f(n, 16, 256, 256, cplx, bufs, True, 0, ctas, C.byref(t)) == 0
+                result["tiles"].append((cplx, n, ctas, t.B, t.smem))
+""")
+    for cplx, n, ctas, B, smem in r["tiles"]:
+        least = 64 // cplx
+        while cplx == 16 and least < 32 and least * n < 32 * 16:
+            least *= 2
+        assert ctas * (smem + 1024) <= 228 * 1024 or B <= least, (cplx, n, ctas, B, smem)
