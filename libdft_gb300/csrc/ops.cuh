@@ -60,26 +60,35 @@ template <class F> int launch_each(size_t n, F f, double bytes = 0.0, const char
   return DFTGPU_OK;
 }
 
-// The (x, y) rows of an [nx][ny][nz] grid, threads along z, a row of more
-// than 256 values in equal segments (blockIdx.z): the lambda gets f(x, y, z, i)
-// with i the linear index, no index division.  Few rows (1-D grids: one) are
-// cut into segments of 32 values, one warp each, so that they use many SMs: a
+// The (x, y) rows of an [nx][ny][nz] grid, threads along z: the lambda gets
+// f(x, y, z, i) with i the linear index, no index division.  A row of more
+// than 256 values runs in equal segments: one after the other in its CTA
+// where the rows alone give every SM eight CTAs (a CTA for each segment takes
+// the rows' halves one pass of the grid after the other; plain FP32 energy
+// density, us, loop / segments: 384^3 1197 / 1265, 256 x 256 x 288 465 / 518),
+// else each in a CTA (blockIdx.z).  Few rows (1-D grids: one) are cut into
+// segments of 32 values, one warp each, so that they use many SMs: a
 // 4096-point row's second OT pass took 150 us on one SM.
 // Short rows share a CTA (up to 256 threads) while that leaves four CTAs per SM.
 struct RowShape { dim3 grid, block; };
 inline RowShape row_shape(int nx, int ny, int nz) {
+  const size_t rows = (size_t) nx * ny, sms = rt().num_sms;
   int nseg = (nz + 255) / 256;
-  if ((size_t) nx * ny * nseg < (size_t) 2 * rt().num_sms) nseg = (nz + 31) / 32;
+  if (rows * nseg < 2 * sms) nseg = (nz + 31) / 32;
   const int bd = ((nz + nseg - 1) / nseg + 31) / 32 * 32;
-  nseg = (nz + bd - 1) / bd;
+  nseg = rows >= 8 * sms ? 1 : (nz + bd - 1) / bd;
   int ry = 1;
-  while (2 * ry * bd <= 256 && (size_t) nx * nseg * ((ny + 2 * ry - 1) / (2 * ry)) >= (size_t) 4 * rt().num_sms) ry *= 2;
+  while (2 * ry * bd <= 256 && (size_t) nx * nseg * ((ny + 2 * ry - 1) / (2 * ry)) >= 4 * sms) ry *= 2;
   return RowShape{ dim3((ny + ry - 1) / ry, nx, nseg), dim3(bd, ry) };
+}
+template <class F> __device__ __forceinline__ void rows_body(int ny, int nz, F &f) {
+  const int y = blockIdx.x * blockDim.y + threadIdx.y, x = blockIdx.y;
+  if (y >= ny) return;
+  for (int z = blockIdx.z * blockDim.x + threadIdx.x; z < nz; z += gridDim.z * blockDim.x) f(x, y, z, (x * ny + y) * nz + z);
 }
 template <class F> __global__ void rows_kernel(int ny, int nz, F f) {
   pdl_begin();
-  const int y = blockIdx.x * blockDim.y + threadIdx.y, x = blockIdx.y, z = blockIdx.z * blockDim.x + threadIdx.x;
-  if (y < ny && z < nz) f(x, y, z, (x * ny + y) * nz + z);
+  rows_body(ny, nz, f);
 }
 
 template <class F> int launch_rows(int nx, int ny, int nz, F f, double bytes = 0.0, const char *name = "pointwise") {
@@ -94,8 +103,7 @@ template <class F> int launch_rows(int nx, int ny, int nz, F f, double bytes = 0
 // for latency-bound passes with many independent loads per element.
 template <int MINB, class F> __global__ void __launch_bounds__(256, MINB) rows_kernel_b(int ny, int nz, F f) {
   pdl_begin();
-  const int y = blockIdx.x * blockDim.y + threadIdx.y, x = blockIdx.y, z = blockIdx.z * blockDim.x + threadIdx.x;
-  if (y < ny && z < nz) f(x, y, z, (x * ny + y) * nz + z);
+  rows_body(ny, nz, f);
 }
 template <int MINB, class F>
 int launch_rows_b(int nx, int ny, int nz, F f, double bytes = 0.0, const char *name = "pointwise") {

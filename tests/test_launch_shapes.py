@@ -104,3 +104,24 @@ for cplx in (8, 16):
         while cplx == 16 and least < 32 and least * n < 32 * 16:
             least *= 2
         assert ctas * (smem + 1024) <= 228 * 1024 or B <= least, (cplx, n, ctas, B, smem)
+
+
+def test_long_rows_stay_in_a_cta(run):
+    """Pointwise passes of grids with many rows longer than 256 values: one CTA takes a whole row."""
+    r = run("""
+G.check(G.lib().dftgpu_init(0), "init")
+for shape in ((64, 64, 384), (64, 64, 512), (40, 48, 1000), (2, 4, 1024)):
+    w, P = G.Wf(shape, 0.8), G.CGrid(shape, 0.8)
+    G.lib().grid_wf_boundary(w.ptr, None, 1e-4, 0.003, 0, shape[0], 0, shape[1], 8, shape[2] - 8)
+    fake.fake_reset()
+    G.lib().grid_wf_absorb_potential(w.ptr, P.ptr, 1e-4, 0.003)
+    G.check(what="absorb")
+    result[str(shape)] = launches()
+""")
+    for case, launches in r.items():
+        assert len(launches) == 1 and launches[0]["bx"] % 32 == 0, (case, launches)
+        l = launches[0]
+        if case == "(2, 4, 1024)":
+            assert l["gz"] * l["bx"] == 1024 and l["bx"] == 32
+        else:
+            assert l["gz"] == 1 and l["gx"] * l["by"] >= 48 and l["bx"] <= 256, (case, l)
