@@ -225,11 +225,19 @@ void set_error(int code, const char *fmt, ...);
 
 // ------------------------------------------------------------------ launches
 // Kernels of the step are launched with programmatic stream serialization:
-// the next kernel's CTAs may become resident while the last CTAs of this one
-// run, and each waits (griddepcontrol.wait: for the completion of everything
-// before it in the stream) before it touches memory that another kernel
-// writes.  Every kernel launched by launch_pdl() calls pdl_begin(), or its two
-// halves with only parameters, constant tables and shared memory between.
+// once every CTA of this kernel has triggered or ended, the next kernel's CTAs
+// become resident where there is room, and each waits (griddepcontrol.wait:
+// for the completion of everything before it in the stream) before it touches
+// memory that another kernel writes.  Every kernel launched by launch_pdl()
+// calls pdl_wait(), with only parameters, constant tables and shared memory
+// before it.  The trigger comes first (pdl_begin()) or late: CTAs placed while
+// this kernel still fills most SMs leave the next one's work unevenly spread,
+// which costs the passes that are bound by each SM's FP64 pipe more than the
+// launch latency that it hides.  So the generic r2c, c2r and convolution passes
+// trigger before their last stage, pointwise passes and reductions at their
+// end; the others first.  Full / plain potential, launched singly, us, all
+// first / so: FP64 48^3 320 / 274 and 124 / 93, 60^3 612 / 551 and 231 / 186,
+// FP32 64^3 88 / 82 and 46 / 38.
 // Under stream capture the launches are ordinary: a graph's kernel-to-kernel
 // edges are the faster ones for small grids.  One predict-correct step, us,
 // ordinary / programmatic: 64^3 FP32 plain launched singly 179 / 142, replayed

@@ -423,8 +423,9 @@ __device__ __forceinline__ void run_stage(int R, const Tile &g, int ef, int p,
 // Forward FFT of the tile: first stage from rd (ef0), the others from shared
 // memory, the last one into wr (efl) when DIRECT (two stages or more), else
 // the result stays in shared memory and its buffer is returned.  Writes
-// alternate between b0 (first) and b1.
-template <bool DIRECT, typename T, class Rd, class Wr>
+// alternate between b0 (first) and b1.  TRIG: the next kernel may start before
+// the last stage (launch_pdl()).
+template <bool DIRECT, typename T, bool TRIG = false, class Rd, class Wr>
 __device__ __forceinline__ typename cplx_t<T>::type *tile_fft(const FftPlan<T> &pl, const Tile &g, int ef0, int efl,
                                                               typename cplx_t<T>::type *b0,
                                                               typename cplx_t<T>::type *b1, const Rd &rd, const Wr &wr) {
@@ -440,6 +441,7 @@ __device__ __forceinline__ typename cplx_t<T>::type *tile_fft(const FftPlan<T> &
   for (int st = 1; st < pl.nst; st++) {
     const int R = pl.radix[st];
     const bool direct = DIRECT && st == pl.nst - 1;
+    if (TRIG && direct) pdl_trigger();
     run_stage<false, T>(R, g, direct ? efl : ef0, p, pl.tw, [&](int l, int e) { return in[g.at(l, e)]; },
                         [&](int l, int e, C v) { if (direct) wr(l, e, v); else out[g.at(l, e)] = v; });
     if (!direct) __syncthreads();
@@ -496,7 +498,8 @@ __global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 3 : 2)
   C *buf0 = reinterpret_cast<C *>(smem_raw), *buf1 = buf0 + args.B * g.LP;
   const FftPlan<T> &pl = args.plan;
   auto none = [](int, int, C) {};
-  pdl_begin();
+  if (MODE == LINE_C2C) pdl_trigger();
+  pdl_wait();
 
   if constexpr (MODE == LINE_C2R) {
     // Z[k] = sum + i w^-k dif, sum, dif = X[k] +- X*[n-k], w = exp(-2 pi i / 2n),
@@ -518,8 +521,8 @@ __global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 3 : 2)
     }
     __syncthreads();
     auto wr = [&](int l, int e, C v) { st(a, b0 + l, e, swap_ri(v)); };
-    C *r = tile_fft<true, T>(pl, g, args.e_fast, args.e_fast_store, buf1, buf0,
-                             [&](int l, int e) { return buf0[g.at(l, e)]; }, wr);
+    C *r = tile_fft<true, T, true>(pl, g, args.e_fast, args.e_fast_store, buf1, buf0,
+                                   [&](int l, int e) { return buf0[g.at(l, e)]; }, wr);
     if (pl.nst > 1) return;
     const FastDiv byn(n);
     for (int idx = threadIdx.x; idx < n * args.B; idx += blockDim.x) {
@@ -529,6 +532,7 @@ __global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 3 : 2)
     }
   } else if constexpr (MODE == LINE_R2C) {
     C *r = tile_fft<false, T>(pl, g, args.e_fast, 0, buf0, buf1, [&](int l, int e) { return ld(a, b0 + l, e); }, none);
+    pdl_trigger();
     // X[k] = (sum - i w^k dif) / 2, sum, dif = Z[k] +- Z*[n-k], and
     // X[n-k] = conj(sum - X[k]), k = 0..n/2
     const int np = n / 2 + 1;
@@ -631,7 +635,7 @@ __global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 3 : 2) xconv_ker
   const int tile = A.B * g.LP, ns = A.plan.nst;
   C *X = reinterpret_cast<C *>(smem_raw), *W = X + tile, *V = W + (ns >= 3 ? tile : 0), *ACC = V + tile;
   const size_t off = (size_t) kz * A.nx * A.ny + y0;
-  pdl_begin();
+  pdl_wait();
   const bool odd = (ns & 1) || ns == 0;   // the number of stage writes: the forward result ends in X
   auto none = [](int, int, C) {};
   int cur = -1;
@@ -660,6 +664,7 @@ __global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 3 : 2) xconv_ker
   };
   for (int o = A.split ? blockIdx.z : 0; o < (A.split ? (int) blockIdx.z + 1 : A.nout); o++) {
     const XOut<T> &out = A.out[o];
+    if (A.split || o == A.nout - 1) pdl_trigger();
     if (out.nt == 1) {
       const XTerm<T> &tm = A.term[out.t0];
       forward(tm.in);

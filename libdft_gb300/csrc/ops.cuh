@@ -8,7 +8,7 @@ namespace dftgpu {
 
 // grid-stride elementwise launch of a device lambda f(i), i < n
 template <class F> __global__ void each_kernel(size_t n, F f) {
-  pdl_begin();
+  pdl_wait();
   for (size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t) gridDim.x * blockDim.x) f(i);
 }
 
@@ -87,7 +87,7 @@ template <class F> __device__ __forceinline__ void rows_body(int ny, int nz, F &
   for (int z = blockIdx.z * blockDim.x + threadIdx.x; z < nz; z += gridDim.z * blockDim.x) f(x, y, z, (x * ny + y) * nz + z);
 }
 template <class F> __global__ void rows_kernel(int ny, int nz, F f) {
-  pdl_begin();
+  pdl_wait();
   rows_body(ny, nz, f);
 }
 
@@ -102,7 +102,7 @@ template <class F> int launch_rows(int nx, int ny, int nz, F f, double bytes = 0
 // The same with a register budget for MINB resident 256-thread CTAs per SM:
 // for latency-bound passes with many independent loads per element.
 template <int MINB, class F> __global__ void __launch_bounds__(256, MINB) rows_kernel_b(int ny, int nz, F f) {
-  pdl_begin();
+  pdl_wait();
   rows_body(ny, nz, f);
 }
 template <int MINB, class F>
@@ -154,7 +154,7 @@ __device__ __forceinline__ double block_sum(double v) {
 }
 
 template <int NV, class F> __global__ void reduce_partial_kernel(size_t n, F f, double *partial) {
-  pdl_begin();
+  pdl_wait();
   double acc[NV];
 #pragma unroll
   for (int j = 0; j < NV; j++) acc[j] = 0.0;
@@ -175,7 +175,7 @@ template <int NV, class F> __global__ void reduce_partial_kernel(size_t n, F f, 
 struct NoAfter { __device__ void operator()(const double *) const {} };
 template <int NV, class After>
 __global__ void reduce_final_kernel(const double *partial, double *slot, double scale, After after) {
-  pdl_begin();
+  pdl_wait();
   double res[NV];
 #pragma unroll
   for (int j = 0; j < NV; j++) {
