@@ -246,6 +246,11 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_begin() { pdl_trigger(); pdl_wait(); }
 
+// Launches of this thread are ordinary while set (par_for with many items).
+inline bool &ordinary_launches() {
+  static thread_local bool v = false;
+  return v;
+}
 template <class... P, class... A>
 inline void launch_pdl(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args) {
   cudaLaunchConfig_t cfg = {};
@@ -259,7 +264,7 @@ inline void launch_pdl(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cuda
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = cs == cudaStreamCaptureStatusNone ? 1 : 0;
+  cfg.numAttrs = cs == cudaStreamCaptureStatusNone && !ordinary_launches() ? 1 : 0;
   cudaLaunchKernelEx(&cfg, k, P(args)...);   // errors: DFT_CHECK_LAUNCH after it
 }
 

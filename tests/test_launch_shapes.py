@@ -125,3 +125,20 @@ for shape in ((64, 64, 384), (64, 64, 512), (40, 48, 1000), (2, 4, 1024)):
             assert l["gz"] * l["bx"] == 1024 and l["bx"] == 32
         else:
             assert l["gz"] == 1 and l["gx"] * l["by"] >= 48 and l["bx"] <= 256, (case, l)
+
+
+def test_launches_in_many_chunks_are_ordinary(run):
+    """A propagation whose kinetic step runs in more than two chunks a branch launches them without programmatic
+    serialization; in fewer chunks, and outside the branches, with it."""
+    r = run("""
+G.check(G.lib().dftgpu_init(0), "init")
+G.set_precision(G.FP32)
+for shape in ((512, 512, 128), (240, 240, 240), (64, 64, 64)):
+    w, V = G.Wf(shape, 0.8), G.CGrid(shape, 0.8)
+    fake.fake_reset()
+    w.propagate(V, 1.0 + 0j)
+    result[str(shape)] = [l["programmatic"] for l in launches()]
+""")
+    assert r["(512, 512, 128)"] == [1] + 7 * 3 * [0] + [1]
+    assert r["(240, 240, 240)"] == [1] + 3 * 3 * [1] + [1]
+    assert r["(64, 64, 64)"] == 5 * [1]
