@@ -103,9 +103,9 @@ __device__ __forceinline__ void pfa_dft(C *u, T s) {
   }
 }
 
-// R-point DFT in place, natural order; s = -1 forward, +1 inverse.
-// Radices 2, 3, 4, 5, 8 directly; 16 and 9 as 4 x 4 and 3 x 3 with their
-// internal twiddles; 6, 10, 12, 15 as prime-factor pairs.
+// R-point DFT in place, natural order; s = -1 forward, +1 inverse.  Radices 2,
+// 3, 4, 5 directly, 9 as 3 x 3 with its internal twiddles, 6, 10, 12, 15 as
+// prime-factor pairs; a stage of radix 2, 4, 8 or 16 is poly_eval() below.
 template <int R, typename C, typename T>
 __device__ __forceinline__ void small_dft(C *u, T s) {
   if constexpr (R == 2) {
@@ -138,53 +138,6 @@ __device__ __forceinline__ void small_dft(C *u, T s) {
     u[4] = m1 - imul<C, T>(n1, s);
     u[2] = m2 + imul<C, T>(n2, s);
     u[3] = m2 - imul<C, T>(n2, s);
-  } else if constexpr (R == 8) {
-    const T h = (T) 0.70710678118654752440;
-    // radix-2 over stride 4, then two radix-4 with the W8 twiddles
-    C a0 = u[0] + u[4], a1 = u[0] - u[4];
-    C b0 = u[2] + u[6], b1 = u[2] - u[6];
-    C c0 = u[1] + u[5], c1 = u[1] - u[5];
-    C d0 = u[3] + u[7], d1 = u[3] - u[7];
-    // even outputs: 4-point DFT of (a0, c0, b0, d0)
-    C e0 = a0 + b0, e1 = a0 - b0, f0 = c0 + d0, f1 = c0 - d0;
-    u[0] = e0 + f0;
-    u[4] = e0 - f0;
-    u[2] = e1 + imul<C, T>(f1, s);
-    u[6] = e1 - imul<C, T>(f1, s);
-    // odd outputs: 4-point DFT of (a1, W c1, W^2 b1, W^3 d1), W = exp(s i pi/4)
-    C b1w = imul<C, T>(b1, s);                       // W^2 b1
-    C c1w, d1w;
-    c1w.x = h * (c1.x - s * c1.y); c1w.y = h * (c1.y + s * c1.x);      // W c1
-    d1w.x = h * (-d1.x - s * d1.y); d1w.y = h * (-d1.y + s * d1.x);    // W^3 d1
-    C g0 = a1 + b1w, g1 = a1 - b1w, k0 = c1w + d1w, k1 = c1w - d1w;
-    u[1] = g0 + k0;
-    u[5] = g0 - k0;
-    u[3] = g1 + imul<C, T>(k1, s);
-    u[7] = g1 - imul<C, T>(k1, s);
-  } else if constexpr (R == 16) {
-    // 4 x 4: 4-point DFTs over n1 of x[4 n1 + n2], twiddles W16^(n2 k1),
-    // 4-point DFTs over n2; X[k1 + 4 k2]
-    const T c1 = (T) 0.923879532511286756128, s1 = (T) 0.382683432365089771728, h = (T) 0.707106781186547524401;
-    C y[4][4];
-#pragma unroll
-    for (int n2 = 0; n2 < 4; n2++) {
-#pragma unroll
-      for (int n1 = 0; n1 < 4; n1++) y[n2][n1] = u[4 * n1 + n2];
-      small_dft<4, C, T>(y[n2], s);
-    }
-    y[1][1] = rot_cs<C, T>(y[1][1], c1, s1, s); y[1][2] = rot_cs<C, T>(y[1][2], h, h, s);
-    y[1][3] = rot_cs<C, T>(y[1][3], s1, c1, s);
-    y[2][1] = rot_cs<C, T>(y[2][1], h, h, s); y[2][2] = imul<C, T>(y[2][2], s);
-    y[2][3] = rot_cs<C, T>(y[2][3], -h, h, s);
-    y[3][1] = rot_cs<C, T>(y[3][1], s1, c1, s); y[3][2] = rot_cs<C, T>(y[3][2], -h, h, s);
-    y[3][3] = rot_cs<C, T>(y[3][3], -c1, -s1, s);
-#pragma unroll
-    for (int k1 = 0; k1 < 4; k1++) {
-      C z[4] = { y[0][k1], y[1][k1], y[2][k1], y[3][k1] };
-      small_dft<4, C, T>(z, s);
-#pragma unroll
-      for (int k2 = 0; k2 < 4; k2++) u[k1 + 4 * k2] = z[k2];
-    }
   } else if constexpr (R == 9) {
     // 3 x 3 with twiddles W9^(n2 k1): (n2, k1) = (1,1), (1,2), (2,1): m = 1, 2; (2,2): m = 4
     const T ca = (T) 0.766044443118978035202, sa = (T) 0.642787609686539326323;
@@ -816,7 +769,10 @@ const DevLimits &dev_limits();
 int choose_tile(int n, int big, int na, int nb, size_t cplx_bytes, int nbufs, bool strided, size_t table, int ctas, TileShape *t);
 inline int line_bufs(int mode, int nst) { return mode == LINE_C2C ? (nst >= 3 ? 2 : 1) : 2; }
 
-constexpr double kBatchBytes = 48e6;   // FP32 spectra of one launch: less than half of L2
+// FP32 spectra up to this size stay in L2 between the passes of a convolution
+// (less than half of it): above it the x pass takes its inputs one after the
+// other (launch_xconv) and the planes run in two halves (convolve).
+constexpr double kBatchBytes = 48e6;
 
 // One launch of the generic line kernel on a given plan and stream.
 template <typename T, int MODE, int NB, class Ld, class St>
