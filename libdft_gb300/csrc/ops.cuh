@@ -76,7 +76,10 @@ template <class F> int launch_each(size_t n, F f, double bytes = 0.0, const char
 // segments of 32 values, one warp each, so that they use many SMs: a
 // 4096-point row's second OT pass took 150 us on one SM.
 // Short rows share a CTA (up to 256 threads) while that leaves four CTAs per SM.
-struct RowShape { dim3 grid, block; };
+struct RowShape {
+  dim3 grid, block;
+  bool loops(int nz) const { return (int) (grid.z * block.x) < nz; }
+};
 inline RowShape row_shape(int nx, int ny, int nz) {
   const size_t rows = (size_t) nx * ny, sms = rt().num_sms;
   int nseg = (nz + 255) / 256;
@@ -87,35 +90,43 @@ inline RowShape row_shape(int nx, int ny, int nz) {
   while (2 * ry * bd <= 256 && (size_t) nx * nseg * ((ny + 2 * ry - 1) / (2 * ry)) >= 4 * sms) ry *= 2;
   return RowShape{ dim3((ny + ry - 1) / ry, nx, nseg), dim3(bd, ry) };
 }
-template <class F> __device__ __forceinline__ void rows_body(int ny, int nz, F &f) {
+// LOOP: the CTA runs its row's segments one after the other (nz > blockDim.x,
+// gridDim.z = 1).  A kernel of its own: the loop costs the others 2 to 6 %.
+template <bool LOOP, class F> __device__ __forceinline__ void rows_body(int ny, int nz, F &f) {
   const int y = blockIdx.x * blockDim.y + threadIdx.y, x = blockIdx.y;
-  if (y >= ny) return;
-  for (int z = blockIdx.z * blockDim.x + threadIdx.x; z < nz; z += gridDim.z * blockDim.x) f(x, y, z, (x * ny + y) * nz + z);
+  if (LOOP) {
+    for (int z = threadIdx.x; z < nz; z += blockDim.x) f(x, y, z, (x * ny + y) * nz + z);
+  } else {
+    const int z = blockIdx.z * blockDim.x + threadIdx.x;
+    if (y < ny && z < nz) f(x, y, z, (x * ny + y) * nz + z);
+  }
 }
-template <class F> __global__ void rows_kernel(int ny, int nz, F f) {
+template <bool LOOP, class F> __global__ void rows_kernel(int ny, int nz, F f) {
   pdl_wait();
-  rows_body(ny, nz, f);
+  rows_body<LOOP>(ny, nz, f);
 }
 
 template <class F> int launch_rows(int nx, int ny, int nz, F f, double bytes = 0.0, const char *name = "pointwise") {
   const RowShape r = row_shape(nx, ny, nz);
   ProfScope prof(name, bytes);
-  launch_pdl(rows_kernel<F>, r.grid, r.block, 0, rt().stream, ny, nz, f);
+  auto k = r.loops(nz) ? rows_kernel<true, F> : rows_kernel<false, F>;
+  launch_pdl(k, r.grid, r.block, 0, rt().stream, ny, nz, f);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }
 
 // The same with a register budget for MINB resident 256-thread CTAs per SM:
 // for latency-bound passes with many independent loads per element.
-template <int MINB, class F> __global__ void __launch_bounds__(256, MINB) rows_kernel_b(int ny, int nz, F f) {
+template <int MINB, bool LOOP, class F> __global__ void __launch_bounds__(256, MINB) rows_kernel_b(int ny, int nz, F f) {
   pdl_wait();
-  rows_body(ny, nz, f);
+  rows_body<LOOP>(ny, nz, f);
 }
 template <int MINB, class F>
 int launch_rows_b(int nx, int ny, int nz, F f, double bytes = 0.0, const char *name = "pointwise") {
   const RowShape r = row_shape(nx, ny, nz);
   ProfScope prof(name, bytes);
-  launch_pdl(rows_kernel_b<MINB, F>, r.grid, r.block, 0, rt().stream, ny, nz, f);
+  auto k = r.loops(nz) ? rows_kernel_b<MINB, true, F> : rows_kernel_b<MINB, false, F>;
+  launch_pdl(k, r.grid, r.block, 0, rt().stream, ny, nz, f);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }
