@@ -142,3 +142,19 @@ for shape in ((512, 512, 128), (240, 240, 240), (64, 64, 64)):
     assert r["(512, 512, 128)"] == [1] + 7 * 3 * [0] + [1]
     assert r["(240, 240, 240)"] == [1] + 3 * 3 * [1] + [1]
     assert r["(64, 64, 64)"] == 5 * [1]
+
+
+def test_large_reductions_are_launched_ordinarily(run):
+    """The partial sums of a reduction over 2^20 terms or more (its last launch but one) start when everything before
+    them has ended, on empty SMs; smaller ones programmatically."""
+    r = run("""
+G.check(G.lib().dftgpu_init(0), "init")
+G.set_precision(G.FP32)
+for shape in ((128, 128, 128), (64, 64, 64)):
+    w = G.Wf(shape, 0.8)
+    fake.fake_reset()
+    G.lib().grid_wf_kinetic_energy(w.ptr)
+    result[str(shape)] = [l["programmatic"] for l in launches()]
+""")
+    assert r["(128, 128, 128)"] == [1, 1, 1, 0, 1]
+    assert r["(64, 64, 64)"] == 5 * [1]
