@@ -66,67 +66,53 @@ template <class F> int launch_each(size_t n, F f, double bytes = 0.0, const char
   return DFTGPU_OK;
 }
 
-// The (x, y) rows of an [nx][ny][nz] grid, threads along z: the lambda gets
-// f(x, y, z, i) with i the linear index, no index division.  A row of more
-// than 256 values runs in equal segments: one after the other in its CTA
-// where the rows alone give every SM eight CTAs (a CTA for each segment takes
-// the rows' halves one pass of the grid after the other; plain FP32 energy
-// density, us, loop / segments: 384^3 1197 / 1265, 256 x 256 x 288 465 / 518),
-// else each in a CTA (blockIdx.z).  Few rows (1-D grids: one) are cut into
-// segments of 32 values, one warp each, so that they use many SMs: a
-// 4096-point row's second OT pass took 150 us on one SM.
+// The (x, y) rows of an [nx][ny][nz] grid, threads along z, a row of more
+// than 256 values in equal segments of one CTA each: the lambda gets
+// f(x, y, z, i) with i the linear index, no index division.  A row's segments
+// are neighbours in the grid (blockIdx.x), so that they run together and the
+// pass goes through memory once: with the segments outermost, plain FP32
+// energy density, us, neighbours / outermost: 384^3 1144 / 1265.  Few rows
+// (1-D grids: one) are cut into segments of 32 values, one warp each, so that
+// they use many SMs: a 4096-point row's second OT pass took 150 us on one SM.
 // Short rows share a CTA (up to 256 threads) while that leaves four CTAs per SM.
-struct RowShape {
-  dim3 grid, block;
-  bool loops(int nz) const { return (int) (grid.z * block.x) < nz; }
-};
+struct RowShape { dim3 grid, block; };
 inline RowShape row_shape(int nx, int ny, int nz) {
-  const size_t rows = (size_t) nx * ny, sms = rt().num_sms;
   int nseg = (nz + 255) / 256;
-  if (rows * nseg < 2 * sms) nseg = (nz + 31) / 32;
+  if ((size_t) nx * ny * nseg < (size_t) 2 * rt().num_sms) nseg = (nz + 31) / 32;
   const int bd = ((nz + nseg - 1) / nseg + 31) / 32 * 32;
-  nseg = rows >= 8 * sms ? 1 : (nz + bd - 1) / bd;
+  nseg = (nz + bd - 1) / bd;
   int ry = 1;
-  while (2 * ry * bd <= 256 && (size_t) nx * nseg * ((ny + 2 * ry - 1) / (2 * ry)) >= 4 * sms) ry *= 2;
-  return RowShape{ dim3((ny + ry - 1) / ry, nx, nseg), dim3(bd, ry) };
+  while (2 * ry * bd <= 256 && (size_t) nx * nseg * ((ny + 2 * ry - 1) / (2 * ry)) >= (size_t) 4 * rt().num_sms) ry *= 2;
+  return RowShape{ dim3(nseg, (ny + ry - 1) / ry, nx), dim3(bd, ry) };
 }
-// LOOP: the CTA runs its row's segments one after the other (nz > blockDim.x,
-// gridDim.z = 1).  A kernel of its own: the loop costs the others 2 to 6 %.
-template <bool LOOP, class F> __device__ __forceinline__ void rows_body(int ny, int nz, F &f) {
-  const int y = blockIdx.x * blockDim.y + threadIdx.y, x = blockIdx.y;
-  if (LOOP) {
-    for (int z = threadIdx.x; z < nz; z += blockDim.x) f(x, y, z, (x * ny + y) * nz + z);
-  } else {
-    const int z = blockIdx.z * blockDim.x + threadIdx.x;
-    if (y < ny && z < nz) f(x, y, z, (x * ny + y) * nz + z);
-  }
+template <class F> __device__ __forceinline__ void rows_body(int ny, int nz, F &f) {
+  const int y = blockIdx.y * blockDim.y + threadIdx.y, x = blockIdx.z, z = blockIdx.x * blockDim.x + threadIdx.x;
+  if (y < ny && z < nz) f(x, y, z, (x * ny + y) * nz + z);
 }
-template <bool LOOP, class F> __global__ void rows_kernel(int ny, int nz, F f) {
+template <class F> __global__ void rows_kernel(int ny, int nz, F f) {
   pdl_wait();
-  rows_body<LOOP>(ny, nz, f);
+  rows_body(ny, nz, f);
 }
 
 template <class F> int launch_rows(int nx, int ny, int nz, F f, double bytes = 0.0, const char *name = "pointwise") {
   const RowShape r = row_shape(nx, ny, nz);
   ProfScope prof(name, bytes);
-  auto k = r.loops(nz) ? rows_kernel<true, F> : rows_kernel<false, F>;
-  launch_pdl(k, r.grid, r.block, 0, rt().stream, ny, nz, f);
+  launch_pdl(rows_kernel<F>, r.grid, r.block, 0, rt().stream, ny, nz, f);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }
 
 // The same with a register budget for MINB resident 256-thread CTAs per SM:
 // for latency-bound passes with many independent loads per element.
-template <int MINB, bool LOOP, class F> __global__ void __launch_bounds__(256, MINB) rows_kernel_b(int ny, int nz, F f) {
+template <int MINB, class F> __global__ void __launch_bounds__(256, MINB) rows_kernel_b(int ny, int nz, F f) {
   pdl_wait();
-  rows_body<LOOP>(ny, nz, f);
+  rows_body(ny, nz, f);
 }
 template <int MINB, class F>
 int launch_rows_b(int nx, int ny, int nz, F f, double bytes = 0.0, const char *name = "pointwise") {
   const RowShape r = row_shape(nx, ny, nz);
   ProfScope prof(name, bytes);
-  auto k = r.loops(nz) ? rows_kernel_b<MINB, true, F> : rows_kernel_b<MINB, false, F>;
-  launch_pdl(k, r.grid, r.block, 0, rt().stream, ny, nz, f);
+  launch_pdl(rows_kernel_b<MINB, F>, r.grid, r.block, 0, rt().stream, ny, nz, f);
   DFT_CHECK_LAUNCH();
   return DFTGPU_OK;
 }
