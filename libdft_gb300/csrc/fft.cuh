@@ -415,15 +415,16 @@ template <typename C> __device__ __forceinline__ C swap_if(C v, bool s) {
 // FP32 forms t first and both elements from it (14 and 12 operations): added
 // into chains of FMAs on the sums, and the second element from the first, the
 // small high-k element of a smooth field's line takes the rounding errors of the
-// large low-k one.  FP64, bound by its operations, runs the chains (12 and 10)
-// but for k = 0, whose partner is the Nyquist element.  Error of the high-k half
-// of a smooth line, chains throughout / so: FP32 n = 16 8.9e-5 / 6.1e-5, 128
-// 8.6e-5 / 8.1e-5, FP64 n = 32 1.55e-13 / 1.29e-13, 128 1.71e-13 / 1.51e-13; FP64
-// with t first everywhere is as accurate and 1 % of a 128^3 step slower.
+// large low-k one.  FP64, bound by its operations, runs the chains (12 and 10).
+// The Nyquist element, k = 0's partner, is stored by itself in both (its value
+// by pair_r2c() is not used).  Error of the high-k half of a smooth line, chains
+// throughout / so: FP32 n = 16 8.9e-5 / 6.1e-5, 128 8.6e-5 / 8.1e-5, FP64 n = 32
+// 1.55e-13 / 1.29e-13, 128 1.71e-13 / 1.51e-13.  (FP64 with t first everywhere is
+// as accurate, and 1 % of a 128^3 step slower.)
 template <typename C> struct CPair { C a, b; };
 template <typename T>
-__device__ __forceinline__ CPair<typename cplx_t<T>::type> pair_r2c(T sx, T sy, T dx, T dy, typename cplx_t<T>::type w, bool k0) {
-  if (sizeof(T) == 4 || k0) {
+__device__ __forceinline__ CPair<typename cplx_t<T>::type> pair_r2c(T sx, T sy, T dx, T dy, typename cplx_t<T>::type w) {
+  if (sizeof(T) == 4) {
     const T hx = (T) 0.5 * w.x, hy = (T) 0.5 * w.y;
     const T tx = fma_t(dx, hy, dy * hx), ty = fma_t(dy, hy, -(dx * hx));
     return { mk<T>(fma_t((T) 0.5, sx, tx), fma_t((T) 0.5, sy, ty)), mk<T>(fma_t((T) 0.5, sx, -tx), fma_t((T) -0.5, sy, ty)) };
@@ -526,9 +527,13 @@ __global__ void __launch_bounds__(FFT_THREADS, sizeof(T) == 4 ? 3 : 2)
       if (l >= g.nl) continue;
       const C zk = r[g.at(l, k)], zm = r[g.at(l, k == 0 ? 0 : n - k)], w = __ldg(&args.tw2[k]);
       const T sx = zk.x + zm.x, sy = zk.y - zm.y, dx = zk.x - zm.x, dy = zk.y + zm.y;
-      const CPair<C> x = pair_r2c<T>(sx, sy, dx, dy, w, k == 0);
+      const CPair<C> x = pair_r2c<T>(sx, sy, dx, dy, w);
       st(a, b0 + l, k, x.a);
-      if (2 * k != n) st(a, b0 + l, n - k, x.b);
+      if (k > 0 && 2 * k != n) st(a, b0 + l, n - k, x.b);
+    }
+    for (int l = threadIdx.x; l < g.nl; l += blockDim.x) {   // the Nyquist element
+      const C z = r[g.at(l, 0)];
+      st(a, b0 + l, n, mk<T>(z.x - z.y, (T) 0));
     }
   } else {
     const bool inv = args.inverse;
@@ -1042,9 +1047,10 @@ __global__ void split_post_kernel(int n, const typename cplx_t<T>::type *__restr
   if (2 * k > n) return;
   const C zk = Z[k], zm = Z[k == 0 ? 0 : n - k], w = __ldg(&tw2[k]);
   const T sx = zk.x + zm.x, sy = zk.y - zm.y, dx = zk.x - zm.x, dy = zk.y + zm.y;
-  const CPair<C> x = pair_r2c<T>(sx, sy, dx, dy, w, k == 0);
+  const CPair<C> x = pair_r2c<T>(sx, sy, dx, dy, w);
   st(0, 0, k, x.a);
-  if (2 * k != n) st(0, 0, n - k, x.b);
+  if (k == 0) st(0, 0, n, mk<T>(zk.x - zk.y, (T) 0));
+  else if (2 * k != n) st(0, 0, n - k, x.b);
 }
 
 // Functors of the potential's and the propagation's z passes, which split lines

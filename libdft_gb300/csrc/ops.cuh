@@ -71,7 +71,7 @@ template <class F> int launch_each(size_t n, F f, double bytes = 0.0, const char
 // f(x, y, z, i) with i the linear index, no index division.  A row's segments
 // are neighbours in the grid (blockIdx.x), so that they run together and the
 // pass goes through memory once: with the segments outermost, plain FP32
-// energy density, us, neighbours / outermost: 384^3 1144 / 1265.  Few rows
+// energy density, us, neighbours / outermost: 384^3 1167 / 1256.  Few rows
 // (1-D grids: one) are cut into segments of 32 values, one warp each, so that
 // they use many SMs: a 4096-point row's second OT pass took 150 us on one SM.
 // Short rows share a CTA (up to 256 threads) while that leaves four CTAs per SM.
