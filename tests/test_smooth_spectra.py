@@ -41,3 +41,29 @@ def test_high_k_of_a_smooth_line(gpu, prec, n, bound):
     finally:
         G.set_precision(G.FP64)
     assert np.sqrt(err / norm) <= 1.07 * bound, np.sqrt(err / norm)
+
+
+@pytest.mark.parametrize("n,bound", [(64, 1.010e-7), (128, 1.075e-7), (256, 1.193e-7)])
+def test_round_trip_of_a_smooth_line(gpu, n, bound):
+    """A propagation over no time, forward and back, of a smooth complex line in FP32.  Bounds: emulated with every
+    product rounded before the sums, plus 2.5 % (three standard deviations of the mean are below 1.5 %)."""
+    G = gpu
+    rng = np.random.default_rng(n)
+    G.set_precision(G.FP32)
+    err = norm = 0
+    try:
+        w, V = G.Wf((1, 1, n), 0.8), G.CGrid((1, 1, n), 0.8)
+        V.zero()
+        inv = float(np.float32(1.0 / n)) * n
+        for _ in range(200000 // n):
+            f = (1 + 0.1 * np.cos(2 * np.pi * np.arange(n) / n + rng.standard_normal())) * (1 + 1e-3 * rng.standard_normal(n))
+            x = (f * (1 + 0.3j)).astype(np.complex64).astype(np.complex128).reshape(1, 1, n)
+            w.set(x)
+            w.propagate(V, 0j)
+            err += np.sum(np.abs(w.get() / inv - x) ** 2)
+            norm += np.sum(np.abs(x) ** 2)
+        V.free()
+        w.free()
+    finally:
+        G.set_precision(G.FP64)
+    assert np.sqrt(err / norm) <= 1.025 * bound, np.sqrt(err / norm)
