@@ -191,12 +191,13 @@ __global__ void reduce_final_kernel(const double *partial, double *slot, double 
   if (threadIdx.x == 0) after(res);
 }
 
-// From four terms a thread on the partial sums are launched ordinarily: their
+// From twelve terms a thread on the partial sums are launched ordinarily: their
 // CTAs take equal shares, and placed while the kernel before them still runs
 // some SMs get eight of them where seven is the even number.  Kinetic energy,
-// FP32, us, programmatic / ordinary: 256^3 652 / 591, 384^3 2441 / 2230, 128^3
-// 107 / 101; 64^3 35.1 / 37.2.
-constexpr size_t kOrdinaryReduce = 4 * (size_t) RED_BLOCKS * RED_THREADS;
+// FP32, us, programmatic / ordinary: 160^3 193 / 179, 256^3 652 / 591, 384^3 2441
+// / 2230, 128^3 107 / 101; 64^3 35.1 / 37.2; but the FP64 energy report of 128^3
+// 5349 / 5372.
+constexpr size_t kOrdinaryReduce = 12 * (size_t) RED_BLOCKS * RED_THREADS;
 
 // f(i, double v[NV]); results (times scale) to slot[0..NV) on the device.
 template <int NV, class F, class After = NoAfter>

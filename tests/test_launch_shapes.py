@@ -143,16 +143,16 @@ for shape in ((512, 512, 128), (240, 240, 240), (64, 64, 64)):
 
 
 def test_large_reductions_are_launched_ordinarily(run):
-    """The partial sums of a reduction over 2^20 terms or more (its last launch but one) start when everything before
+    """The partial sums of a reduction over 3 * 2^20 terms or more (its last launch but one) start when everything before
     them has ended, on empty SMs; smaller ones programmatically."""
     r = run("""
 G.check(G.lib().dftgpu_init(0), "init")
 G.set_precision(G.FP32)
-for shape in ((128, 128, 128), (64, 64, 64)):
+for shape in ((160, 160, 160), (128, 128, 128)):
     w = G.Wf(shape, 0.8)
     fake.fake_reset()
     G.lib().grid_wf_kinetic_energy(w.ptr)
     result[str(shape)] = [l["programmatic"] for l in launches()]
 """)
-    assert r["(128, 128, 128)"] == [1, 1, 1, 0, 1]
-    assert r["(64, 64, 64)"] == 5 * [1]
+    assert r["(160, 160, 160)"] == [1, 1, 1, 0, 1]
+    assert r["(128, 128, 128)"] == 5 * [1]
