@@ -189,7 +189,7 @@ __device__ __forceinline__ void small_dft(C *u, T s) {
 // pi/8 are below the circle, radix 5 above it): with every c1 as it rounds
 // radix 16 lowers it by 2.7e-8, with one of the four rounded up by 2.0e-8,
 // which brings lengths 240, 160 and 80 from -2.1e-8, -9.1e-9 and -5.3e-9 to
-// -1.3e-8, -2.3e-9 and 1e-9 (all four up: 80 and 160 at +2e-8).
+// -1.4e-8, -2.3e-9 and below 1e-9 (all four up: 80 and 160 at +2e-8).
 __device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
 
@@ -465,7 +465,8 @@ template <typename T> struct LineArgs {
 // one's store straight to it, a line crosses shared memory only between
 // stages (n <= 256: once; the staged form it replaces wrote and read it once
 // more at either end and twice per stage).  Inverse transforms run the
-// forward stages on (im, re).  The R2C / C2R steps take k and n - k together.  The last tile may be partial.
+// forward stages on (im, re).  The R2C / C2R steps take k and n - k together.
+// The last tile may be partial.
 // FP64 is bound by its issue rate of 2 operations per clock and SM, whatever
 // the occupancy, so what counts is operations per element: 22 at n = 128 with
 // radices 8, 8, 2 and separate twiddle products, 18 as 16, 8 with the
